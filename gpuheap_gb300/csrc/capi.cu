@@ -83,7 +83,7 @@ gh_status device_error(const gh_heap* h) {
 }
 
 gh::impl::LaunchArgs args_of(const gh_heap* h, cudaStream_t s) {
-    return gh::impl::LaunchArgs{&h->d, threads_of(h), grid_of(h), s, h->opSize};
+    return gh::impl::LaunchArgs{&h->d, threads_of(h), grid_of(h), s, h->opSize, h->blockThreads == 0, h->grid == 0};
 }
 
 // Calls f(K{}) with the heap's key type.

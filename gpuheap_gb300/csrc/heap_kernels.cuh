@@ -32,9 +32,12 @@ struct Desc {
     int ownerDepth;  // owner-mode resident depth: -1 automatic, 0 off, else 2..4
 };
 
-// insertKernel: chunks of `chunk` keys, grid-strided over blocks.
+// insertKernel: chunks of `chunk` keys, grid-strided over blocks.  `rest`:
+// the keys left over by a bulk insert of full batches, which a heap build
+// has inserted already when the heap has a partial buffer.
 template <typename H, typename K>
-__global__ void __launch_bounds__(1024) k_insert(H h, const K* __restrict__ keys, long long n, int chunk) {
+__global__ void __launch_bounds__(1024) k_insert(H h, const K* __restrict__ keys, long long n, int chunk, bool rest) {
+    if (rest && H::kHasPartialBuffer && h.state->build) return;
     const long long nchunks = (n + chunk - 1) / chunk;
     for (long long i = blockIdx.x; i < nchunks; i += gridDim.x) {
         const long long off = i * chunk;
@@ -45,26 +48,101 @@ __global__ void __launch_bounds__(1024) k_insert(H h, const K* __restrict__ keys
     }
 }
 
+// A bulk insert that makes the heap at most this many times the new batches
+// is a heap build (k_build); one that adds fewer batches inserts them one by
+// one (k_insert_reserved).  Measured on GB300, microseconds for m batches
+// into a heap of N (build / one by one): u32, batch 2048, N = 16384: m = 64
+// 264 / 160, m = 256 174 / 462; batch 1024, N = 1024: m = 16 111 / 96,
+// m = 64 87 / 236; batch 256, N = 8192: m = 64 155 / 85, m = 256 109 / 181;
+// u64, batch 1024, N = 4096: m = 16 266 / 123, m = 64 143 / 304.  The lines
+// cross at N / m = 50 to 160.
+constexpr int kBuildRatio = 48;
+
 // Bulk insert of `m` full batches, step 1 (one thread): with the partial
 // buffer empty, no error recorded and room for all of them, reserve targets
 // batchCount+1 .. batchCount+m (batchCount moves past them now, as m
-// node-0 hand-offs would have moved it); otherwise reserve nothing and the
-// insert kernel takes node 0 per batch as the reference does.
+// node-0 hand-offs would have moved it) and choose how to fill them;
+// otherwise reserve nothing and the insert kernel takes node 0 per batch as
+// the reference does.
 static __global__ void k_reserve(HeapState* st, int batchNum, long long m) {
     const int bc = st->batchCount;
     const bool ok = m > 0 && st->err == 0 && st->partialBufferSize == 0 && bc + m <= batchNum;
     st->resvBase = bc;
     st->resvCount = ok ? static_cast<int>(m) : 0;
     st->resvTurn = bc + 1;
+    st->build = ok && bc + m <= kBuildRatio * m;
+    st->buildNext = bc + static_cast<int>(ok ? m : 0);
     if (ok) st->batchCount = bc + static_cast<int>(m);
 }
 
 // Step 2: the reserved targets' lock words take the state an insert holds
 // its target in (top-down TARGET, bottom-up INUSE), so that an insert that
-// reaches one before its own insert has written it waits there.
-static __global__ void k_mark_reserved(const HeapState* st, int* status, int held) {
+// reaches one before its own insert has written it waits there.  A heap
+// build holds (INUSE) every node whose batch it sifts: the targets and
+// their ancestors.
+template <typename H>
+__global__ void k_mark_reserved(const HeapState* st, int* status) {
     const int base = st->resvBase, cnt = st->resvCount;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) status[base + 1 + i] = held;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (!st->build) {
+        const int held = H::kVariant == kTopDown ? TD::TARGET : BU::INUSE;
+        for (int i = t; i < cnt; i += stride) status[base + 1 + i] = held;
+        return;
+    }
+    for (int i = 1 + t; i <= base + cnt; i += stride)
+        if (i > base || H::hasDescendantIn(i, base + 1, base + cnt)) status[i] = H::lockedState();
+}
+
+// Step 3 of a heap build: nodes base + m .. 1 in descending order, each
+// taken by a running block, so a block only waits for nodes that other
+// running blocks hold, whatever the grid.  A new node's batch is loaded and
+// sorted; a node that was there before is sifted again when it has a new
+// one below it.  The work is about one sift step per node (half the nodes
+// are leaves, a quarter sift one level ...) where inserting one by one takes
+// a step per level for each and every path meets at the top.  2^28 u32 keys,
+// batch 2048: 16.3 ms (112 ms one by one); 2^20, batch 1024: 124 us.
+// Bound by the blocks' sort and merge instructions: 4 GiB cross DRAM, 0.6 ms of it.  Node "0" is the ragged last batch (fewer than
+// batchSize keys), which only meets the root and the partial buffer.
+template <typename H, typename K>
+__global__ void __launch_bounds__(1024) k_build(H h, const K* __restrict__ keys, int tail) {
+    HeapState* st = h.state;
+    if (!st->build) return;
+    const int base = st->resvBase, top = base + st->resvCount;
+    const int B = h.batchSize, tid = threadIdx.x;
+    K* s0 = h.region(0);
+    int v;
+    {
+        typename H::Op op(&h, h.ctl(s0));
+        OpCtl* c = op.c;
+        for (;;) {
+            if (tid == 0) {
+                const int err = detail::ld_relaxed(&st->err);
+                const int next = atomicSub(&st->buildNext, 1);
+                c->w[10] = err ? -1 : next;
+            }
+            __syncthreads();
+            v = c->w[10];
+            if (v < 1) break;
+            if (v > base) {
+                const K* src = keys + static_cast<size_t>(v - 1 - base) * B;
+                for (int q = tid; q < B; q += blockDim.x) s0[q] = src[q];
+                __syncthreads();
+                detail::bitonic_sort(s0, B);
+            } else if (H::hasDescendantIn(v, base + 1, top)) {
+                if (tid == 0) {
+                    op.issue(h.nodeBytes());
+                    h.load(s0, v, &c->bar);
+                }
+                if (!op.wait()) break;
+            } else {
+                __syncthreads();  // every thread has read c->w[10]
+                continue;
+            }
+            h.buildNode(op, v, s0, top);
+            __syncthreads();
+        }
+    }
+    if (H::kHasPartialBuffer && v == 0 && tail > 0) h.insertion(keys + static_cast<size_t>(top - base) * B, tail, 0);
 }
 
 // Step 3: insertKernel over the full batches; batch i goes to reserved
@@ -74,6 +152,7 @@ static __global__ void k_mark_reserved(const HeapState* st, int* status, int hel
 template <typename H, typename K>
 __global__ void __launch_bounds__(1024) k_insert_reserved(H h, const K* __restrict__ keys, long long m) {
     const int base = h.state->resvBase, cnt = h.state->resvCount;
+    if (h.state->build) return;
     for (long long i = blockIdx.x; i < m; i += gridDim.x) {
         const K* src = keys + i * h.batchSize;
         if (cnt) h.insertionReserved(src, base + 1 + static_cast<int>(i), 0);
@@ -175,6 +254,8 @@ static __global__ void k_init_state(HeapState* st, int deleteCount) {
         st->resvTurn = 0;
         st->delTicket = 0;
         st->delServing = 0;
+        st->build = 0;
+        st->buildNext = 0;
         st->err = 0;
         st->errOp = 0;
         st->errNode = 0;

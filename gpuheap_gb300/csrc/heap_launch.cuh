@@ -17,6 +17,8 @@ struct LaunchArgs {
     int grid;
     cudaStream_t stream;
     int* opSize;
+    bool autoThreads = false;  // `threads` / `grid` are the heap's automatic choice
+    bool autoGrid = false;
     bool reserve = true;  // bulk inserts of full batches may reserve their targets (k_reserve)
 };
 
@@ -96,8 +98,34 @@ inline H view_of(const Desc& d, int sortOutput) {
     return h;
 }
 
+// Threads of a heap build's blocks (k_build): 8 keys a thread in the merges,
+// so that several blocks share an SM and hide each other's lock and load
+// latency.  Measured on GB300: 2^28 u32, batch 2048: 16.3 ms at 512 threads,
+// 24.3 at 1024; 2^24 u64, batch 1024: 1.15 ms at 256, 1.46 at 512.
+inline int build_threads(int batchSize) { return batchSize >= 128 ? batchSize / 4 : 32; }
+
+// The heap build of m reserved batches (and the `tail` keys after them).
+template <typename K>
+cudaError_t launch_build(const LaunchArgs& a, const K* keys, long long m, int tail) {
+    const int threads = a.autoThreads ? build_threads(a.d->batchSize) : a.threads;
+    return dispatch<K>(*a.d, threads, [&](auto proto) -> cudaError_t {
+        using H = decltype(proto);
+        const H h = view_of<H>(*a.d, 1);
+        const size_t smem = H::smemBytes(a.d->batchSize);
+        const void* fn = reinterpret_cast<const void*>(k_build<H, K>);
+        cudaError_t e = allow_smem<H>(fn, smem);
+        if (e != cudaSuccess) return e;
+        long long g = a.autoGrid ? resident_grid(fn, threads, smem, INT_MAX) : a.grid;
+        if (g == INT_MAX) g = a.grid;
+        k_build<H, K><<<static_cast<int>(g < m ? g : m), threads, smem, a.stream>>>(h, keys, tail);
+        count_launch();
+        return cudaGetLastError();
+    });
+}
+
 // Full batches (chunk == batchSize) go to targets reserved up front when the
-// partial buffer is empty (k_reserve, k_mark_reserved, k_insert_reserved);
+// partial buffer is empty (k_reserve, k_mark_reserved, then k_build or
+// k_insert_reserved);
 // a ragged last chunk, or any other chunk size, goes through insertion().
 template <typename K>
 cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int chunk) {
@@ -112,10 +140,11 @@ cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int c
             if (e != cudaSuccess) return e;
             k_reserve<<<1, 1, 0, a.stream>>>(a.d->state, a.d->batchNum, m);
             count_launch();
-            const int held = a.d->variant == kTopDown ? TD::TARGET : BU::INUSE;
             const long long mb = (m + 255) / 256;
-            k_mark_reserved<<<static_cast<int>(mb < 1024 ? mb : 1024), 256, 0, a.stream>>>(a.d->state, a.d->status, held);
+            k_mark_reserved<H><<<static_cast<int>(mb < 1024 ? mb : 1024), 256, 0, a.stream>>>(a.d->state, a.d->status);
             count_launch();
+            e = launch_build<K>(a, keys, m, H::kHasPartialBuffer ? static_cast<int>(n - m * B) : 0);
+            if (e != cudaSuccess) return e;
             const int g = resident_grid(reinterpret_cast<const void*>(k_insert_reserved<H, K>), a.threads, smem,
                                         static_cast<int>(m < a.grid ? m : a.grid));
             k_insert_reserved<H, K><<<g, a.threads, smem, a.stream>>>(h, keys, m);
@@ -129,7 +158,7 @@ cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int c
         if (e != cudaSuccess) return e;
         const long long nchunks = (rest + chunk - 1) / chunk;
         const int g = static_cast<int>(nchunks < a.grid ? nchunks : a.grid);
-        k_insert<H, K><<<g, a.threads, smem, a.stream>>>(h, keys + m * B, rest, chunk);
+        k_insert<H, K><<<g, a.threads, smem, a.stream>>>(h, keys + m * B, rest, chunk, m > 0);
         count_launch();
         return cudaGetLastError();
     });

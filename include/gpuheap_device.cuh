@@ -85,7 +85,9 @@ struct alignas(128) HeapState {
     int resvTurn;           // top-down reserved inserts take the root in target order: the next target
     int delTicket;          // bulk deletes: next ticket for node 0 (atomicAdd)
     int delServing;         // bulk deletes: the ticket whose holder may lock node 0 now
-    int pad2[9];
+    int build;              // bulk insert: 1 when the reserved targets are filled by a heap build (k_build)
+    int buildNext;          // heap build: next node to take, counting down
+    int pad2[7];
     unsigned long long appStats[8];  // applications: counters (e.g. pops, expansions, relaxations)
 };
 
@@ -709,6 +711,44 @@ struct Heap {
         else insert_bottomup(op, s0, s1, s2, target - 1, parkTag, true);
     }
 
+    // Whether node p has a descendant in [lo, hi] (lo > p).  Top-down: the
+    // descendants of p j levels down are p * 2^j .. (p + 1) * 2^j - 1.
+    // Bottom-up: the parent of 2^L + x is 2^(L-1) + (x mod 2^(L-1)) (parentOf
+    // without the reversals), so the descendants of 2^L + y on a lower level
+    // 2^M.. are the nodes 2^M + x with x = y mod 2^L.
+    __device__ __forceinline__ static bool hasDescendantIn(int p, int lo, int hi) {
+        const int L = 31 - __clz(p);
+        for (int j = 1; L + j < 31; ++j) {
+            const int first = 1 << (L + j);  // of the level
+            if (first > hi) return false;
+            const int last = first + (first - 1) < hi ? first + (first - 1) : hi;
+            if (last < lo) continue;
+            if constexpr (VARIANT == kTopDown) {
+                if ((static_cast<long long>(p) << j) <= last && ((static_cast<long long>(p) + 1) << j) > lo) return true;
+            } else {
+                const int from = (lo > first ? lo : first) - first, m = (1 << L) - 1;
+                if (from + ((p - from) & m) <= last - first) return true;
+            }
+        }
+        return false;
+    }
+
+    // One node of a heap build (Floyd's bottom-up construction on batches):
+    // node v's batch, sorted, is in s0; every node below it up to `limit`
+    // belongs to a heap.  v's lock word is held (INUSE) since before the
+    // build; the batch sifts down from v as a delete's refill does, which
+    // frees v after its first level.  A parent's sift waits there for its
+    // children's lock words, so sifts follow each other down hand over hand.
+    __device__ __forceinline__ void buildNode(Op& op, int v, K* s0, int limit) const {
+        if (leftOf(v) > limit) {
+            store_node(v, s0);
+            __syncthreads();
+            if (threadIdx.x == 0) unlock(v, 0);
+        } else {
+            sift_loop(op, v, 0, s0, s0 + 2 * batchSize, s0 + 3 * batchSize, nullptr, limit);
+        }
+    }
+
     // Top-down path (heap/tditdd/heap.cuh:666-752).  Entered holding node 0;
     // the carried batch is in s0.  Each node on the root -> target path is
     // held while its merge runs; the next node is locked and its load started
@@ -1328,8 +1368,9 @@ struct Heap {
     // `cf` (optional): the carried batch is still in flight on a barrier of
     // its own; the first level takes and loads the children meanwhile, then
     // waits for both (and releases cf->cons once the carried batch is in).
+    // `limit` (optional): nodes above it hold nothing and are not looked at.
     __device__ __forceinline__ void sift_loop(Op& op, int cur, int curPrev, K* C, K* Xc, K* Yc,
-                                              CarriedInFlight* cf = nullptr) const {
+                                              CarriedInFlight* cf = nullptr, int limit = 0x7fffffff) const {
         OpCtl* c = op.c;
         const int tid = threadIdx.x;
         const int B = batchSize;
@@ -1337,8 +1378,8 @@ struct Heap {
             Level lv;
             lv.l = leftOf(cur);
             lv.r = rightOrNone(lv.l);
-            if (tid == lockThread(0)) { int p; c->w[3] = takeChild(lv.l, p); c->w[4] = p; }
-            if (tid == lockThread(1)) { int p; c->w[5] = takeChild(lv.r, p); c->w[6] = p; }
+            if (tid == lockThread(0)) { int p = 0; c->w[3] = lv.l > limit ? kAbsent : takeChild(lv.l, p); c->w[4] = p; }
+            if (tid == lockThread(1)) { int p = 0; c->w[5] = lv.r > limit ? kAbsent : takeChild(lv.r, p); c->w[6] = p; }
             __syncthreads();
             if (c->w[3] < 0 || c->w[5] < 0) {
                 carried_in(cf, c);
