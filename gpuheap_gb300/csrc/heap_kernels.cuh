@@ -100,8 +100,9 @@ __global__ void k_mark_reserved(const HeapState* st, int* status) {
 // one below it.  The work is about one sift step per node (half the nodes
 // are leaves, a quarter sift one level ...) where inserting one by one takes
 // a step per level for each and every path meets at the top.  2^28 u32 keys,
-// batch 2048: 16.3 ms (112 ms one by one); 2^20, batch 1024: 124 us.
-// Bound by the blocks' sort and merge instructions: 4 GiB cross DRAM, 0.6 ms of it.  Node "0" is the ragged last batch (fewer than
+// batch 2048: 5.7 ms (112 ms one by one; 16.3 ms with the batches sorted by
+// a shared-memory bitonic network); 2^20, batch 1024: 91 us.  Bound by the
+// blocks' sort and merge instructions: 4 GiB cross DRAM, 0.6 ms of it.  Node "0" is the ragged last batch (fewer than
 // batchSize keys), which only meets the root and the partial buffer.
 template <typename H, typename K>
 __global__ void __launch_bounds__(1024) k_build(H h, const K* __restrict__ keys, int tail) {
@@ -125,9 +126,7 @@ __global__ void __launch_bounds__(1024) k_build(H h, const K* __restrict__ keys,
             if (v < 1) break;
             if (v > base) {
                 const K* src = keys + static_cast<size_t>(v - 1 - base) * B;
-                for (int q = tid; q < B; q += blockDim.x) s0[q] = src[q];
-                __syncthreads();
-                detail::bitonic_sort(s0, B);
+                h.sortBatch(src, B, s0);
             } else if (H::hasDescendantIn(v, base + 1, top)) {
                 if (tid == 0) {
                     op.issue(h.nodeBytes());

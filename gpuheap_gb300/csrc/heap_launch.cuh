@@ -100,8 +100,8 @@ inline H view_of(const Desc& d, int sortOutput) {
 
 // Threads of a heap build's blocks (k_build): 8 keys a thread in the merges,
 // so that several blocks share an SM and hide each other's lock and load
-// latency.  Measured on GB300: 2^28 u32, batch 2048: 16.3 ms at 512 threads,
-// 24.3 at 1024; 2^24 u64, batch 1024: 1.15 ms at 256, 1.46 at 512.
+// latency.  Measured on GB300: 2^28 u32, batch 2048: 5.7 ms at 512 threads,
+// 10.2 at 1024; 2^24 u64, batch 1024: 0.72 ms at 256, 0.76 at 512.
 inline int build_threads(int batchSize) { return batchSize >= 128 ? batchSize / 4 : 32; }
 
 // The heap build of m reserved batches (and the `tail` keys after them).

@@ -2,8 +2,8 @@
 // can check them in isolation against a sort: the two-batch merge that every
 // insert and sift step uses (merge path per thread, gh::detail::merge_split_t),
 // the owner-mode delete's warp-window merge (ballot split, bitonic network,
-// shared-memory transposes; owner_delete.cuh) and the bitonic sort of an
-// insert batch (gh::detail::bitonic_sort).  The reference tests its
+// shared-memory transposes; owner_delete.cuh) and the sort of an insert batch
+// (gh::detail::sort_batch).  The reference tests its
 // counterparts, imergePath and ibitonicSort (heap/heaputil.cuh:23-47,
 // 99-158), with local_test/merge_path over batch 32..2048 x block
 // 32..min(batch, 1024).
@@ -57,10 +57,7 @@ template <typename K>
 __global__ void __launch_bounds__(1024) k_sort_batch(const K* in, int n, K* out) {
     extern __shared__ __align__(16) unsigned char sm[];
     K* s = reinterpret_cast<K*>(sm);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = in[i];
-    __syncthreads();
-    gh::detail::bitonic_sort(s, n);
-    __syncthreads();
+    gh::detail::sort_batch_rt<K>(in, n, s, n, gh::impl::ow::key_max<K>());
     for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = s[i];
 }
 

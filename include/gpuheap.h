@@ -505,8 +505,8 @@ gh_status gh_gen_grid(int width, int height, unsigned long long seed, int obstac
  * path, 2n / threads keys per thread, 1..16); method 1: the owner-mode
  * delete's warp-window merge (windows of 1024 four-byte or 512 eight-byte
  * keys, so 2n at least one window).  gh_sort_batch: sorts in_dev[0, n) (n a
- * power of two in [2, 8192]) into out_dev with the insert batch's bitonic
- * network.  threads: a power of two in [32, 1024]. */
+ * power of two in [2, 8192]) into out_dev with the sort of an
+ * insert batch.  threads: a power of two in [32, 1024]. */
 gh_status gh_merge_batches(int key_kind, int method, const void* a_dev, const void* b_dev, int n, void* lo_dev,
                            void* hi_dev, int threads, void* stream);
 gh_status gh_sort_batch(int key_kind, const void* in_dev, int n, void* out_dev, int threads, void* stream);

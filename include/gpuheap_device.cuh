@@ -21,8 +21,8 @@
 //     an mbarrier), merged in registers by a merge-path split of two sorted
 //     batches and written straight from registers with 16-byte stores, so a
 //     level step costs one bulk load, one merge and one store;
-//   * the insert batch is sorted by a bitonic network whose short strides run
-//     under __syncwarp instead of __syncthreads;
+//   * the insert batch is sorted in registers, a run per warp, and the runs
+//     merged in shared memory;
 //   * locks use acquire/release atomics at GPU scope (the reference publishes
 //     node data with plain stores); a bulk copy reads a node only after the
 //     lock acquire that follows its writer's fence.acq_rel.gpu + release;
@@ -250,41 +250,46 @@ __device__ __forceinline__ K lds(unsigned addr) {
     }
 }
 
+// Outputs [d, d + IPT) of the merge of the sorted runs at the shared-window
+// addresses sa and sb (n keys each, d + IPT <= 2n): a binary search on the
+// diagonal d finds the split (a wins ties, as heap/heaputil.cuh:99-158
+// does), IPT sequential steps fill the registers.
+template <typename K, int IPT>
+__device__ __forceinline__ void merge_run(unsigned sa, unsigned sb, int n, int d, K (&r)[IPT]) {
+    constexpr unsigned S = sizeof(K);
+    int i0 = d > n ? d - n : 0, i1 = d < n ? d : n;
+    while (i0 < i1) {
+        const int m = (i0 + i1) >> 1;
+        const K x = lds<K>(sa + S * m), y = lds<K>(sb + S * (d - 1 - m));
+        const bool p = x <= y;
+        i0 = p ? m + 1 : i0;
+        i1 = p ? i1 : m;
+    }
+    int i = i0, j = d - i0;
+    K av = lds<K>(sa + S * (i < n ? i : n - 1)), bv = lds<K>(sb + S * (j < n ? j : n - 1));
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const bool ta = (j >= n) || (i < n && av <= bv);
+        r[k] = ta ? av : bv;
+        if (ta) { ++i; av = lds<K>(sa + S * (i < n ? i : n - 1)); }
+        else { ++j; bv = lds<K>(sb + S * (j < n ? j : n - 1)); }
+    }
+}
+
 // Merge-path split of two sorted runs a[0,n) and b[0,n) held in shared
 // memory: the n smallest keys go to lo[0,n), the n largest to hi[0,n) (either
 // may be null to discard; either may be shared or global).  Thread `tid` of
-// the participating group produces outputs [tid*IPT, (tid+1)*IPT): a binary
-// search on its diagonal finds the split (a wins ties, as
-// heap/heaputil.cuh:99-158 does), IPT sequential steps fill registers, a
-// barrier lets lo/hi alias a/b, and the run is stored with vector stores.
+// the participating group produces outputs [tid*IPT, (tid+1)*IPT)
+// (merge_run), a barrier lets lo/hi alias a/b, and the run is stored with
+// vector stores.
 // Every thread of the block must call it (the barrier is block-wide); threads
 // with tid*IPT >= 2n only take part in the barrier.  No trailing barrier.
 template <typename K, int IPT>
 __device__ __forceinline__ void merge_split_t(const K* a, const K* b, K* lo, K* hi, int n, int tid) {
     const int d = tid * IPT;
     const bool active = d < 2 * n;
-    const unsigned sa = smem_u32(a), sb = smem_u32(b);
-    constexpr unsigned S = sizeof(K);
     K r[IPT];
-    if (active) {
-        int i0 = d > n ? d - n : 0, i1 = d < n ? d : n;
-        while (i0 < i1) {
-            const int m = (i0 + i1) >> 1;
-            const K x = lds<K>(sa + S * m), y = lds<K>(sb + S * (d - 1 - m));
-            const bool p = x <= y;
-            i0 = p ? m + 1 : i0;
-            i1 = p ? i1 : m;
-        }
-        int i = i0, j = d - i0;
-        K av = lds<K>(sa + S * (i < n ? i : n - 1)), bv = lds<K>(sb + S * (j < n ? j : n - 1));
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const bool ta = (j >= n) || (i < n && av <= bv);
-            r[k] = ta ? av : bv;
-            if (ta) { ++i; av = lds<K>(sa + S * (i < n ? i : n - 1)); }
-            else { ++j; bv = lds<K>(sb + S * (j < n ? j : n - 1)); }
-        }
-    }
+    if (active) merge_run<K, IPT>(smem_u32(a), smem_u32(b), n, d, r);
     __syncthreads();
     if (active) {
         K* dst = d < n ? (lo ? lo + d : nullptr) : (hi ? hi + (d - n) : nullptr);
@@ -325,6 +330,124 @@ __device__ __forceinline__ void bitonic_sort(K* s, int n) {
             if (j <= 32 && next_j <= 32 && !(j == 1 && k == n)) __syncwarp();
             else __syncthreads();
         }
+    }
+}
+
+// Ascending sort of 32 * R keys in the registers of a warp, key i in m[i % R]
+// of lane i / R: a bitonic network whose merges start by comparing mirrored
+// keys, so every comparator points the same way; strides below R stay inside
+// a lane, the others are shuffles.
+template <typename K, int R>
+__device__ __forceinline__ void warp_sort(K (&m)[R]) {
+    const int lane = static_cast<int>(threadIdx.x) & 31;
+    auto cmpx = [](K& x, K& y) {
+        const K u = x, v = y;
+        const bool in = u <= v;
+        x = in ? u : v;
+        y = in ? v : u;
+    };
+    auto strides_in_lane = [&](int from) {
+#pragma unroll
+        for (int j = R / 2; j > 0; j >>= 1) {
+            if (j > from) continue;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if ((r & j) == 0) cmpx(m[r], m[r + j]);
+        }
+    };
+#pragma unroll
+    for (int k = 2; k <= R; k <<= 1) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if ((r & (k >> 1)) == 0) cmpx(m[r], m[r ^ (k - 1)]);
+        strides_in_lane(k >> 2);
+    }
+#pragma unroll
+    for (int g = 2; g <= 32; g <<= 1) {  // lanes in a merge
+        const bool lower = (lane & (g >> 1)) == 0;
+#pragma unroll
+        for (int r = 0; r < (R + 1) / 2; ++r) {
+            const int q = R - 1 - r;
+            const K x = __shfl_xor_sync(0xffffffffu, m[q], g - 1);
+            const K y = __shfl_xor_sync(0xffffffffu, m[r], g - 1);
+            m[r] = ((m[r] < x) == lower) ? m[r] : x;
+            if (q != r) m[q] = ((m[q] < y) == lower) ? m[q] : y;
+        }
+#pragma unroll
+        for (int j = g >> 2; j > 0; j >>= 1) {
+            const bool low = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const K x = __shfl_xor_sync(0xffffffffu, m[r], j);
+                m[r] = ((m[r] < x) == low) ? m[r] : x;
+            }
+        }
+        strides_in_lane(R >> 1);
+    }
+}
+
+// Sorts src[0, size) ascending into s[0, n) (shared, 16-byte aligned), the
+// rest of s filled with `pad` (not below any key): n a power of two, R keys
+// per thread, n / R <= blockDim.x.  Warps sort runs of 32 * R keys in
+// registers, then the block merges pairs of runs (merge_run) as far as the
+// keys reach.  src may be global or shared, and s itself.  Every thread of
+// the block calls it; ends with a barrier.
+// A shared-memory bitonic network takes log2(n) (log2(n) + 1) / 2 passes over
+// the batch with a barrier each (66 at 2048); here log2(n / (32 R)) merges
+// follow one pass.  Bound by instructions: a heap build of 2^28 u32 keys at
+// batch 2048 takes 5.7 ms with it and 16.3 ms with the network; 24 single
+// operations at batch 256 take 514 us instead of 587.
+template <typename K, int R>
+__device__ __forceinline__ void sort_batch(const K* src, int size, K* s, int n, K pad) {
+    constexpr int run = 32 * R;
+    const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
+    const int base = (tid >> 5) * run;
+    if (base < n) {
+        K m[R];
+        if (base < size) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int i = base + r * 32 + lane;
+                m[r] = i < size ? src[i] : pad;
+            }
+            warp_sort<K, R>(m);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) m[r] = pad;
+        }
+        if (base + lane * R < n) store_run<K, R>(s + base + lane * R, m);
+    }
+    __syncthreads();
+    const unsigned s32 = smem_u32(s);
+    for (int len = run; len < size; len <<= 1) {
+        const int d = tid * R, pair = d & ~(2 * len - 1);
+        const bool active = d < n && pair + len < size;  // the second run holds keys
+        K m[R];
+        if (active) {
+            const unsigned a = s32 + static_cast<unsigned>(pair * sizeof(K));
+            merge_run<K, R>(a, a + static_cast<unsigned>(len * sizeof(K)), len, d - pair, m);
+        }
+        __syncthreads();
+        if (active) store_run<K, R>(s + d, m);
+        __syncthreads();
+    }
+}
+
+// R chosen at run time: the keys a thread has when the block's threads share
+// the batch (1 to 8); more keys a thread, and blocks of less than a warp
+// (the retrieving heap's at batch 16), take the bitonic network.
+template <typename K>
+__device__ __forceinline__ void sort_batch_rt(const K* src, int size, K* s, int n, K pad) {
+    const int per = blockDim.x < 32 ? 16 : n / static_cast<int>(blockDim.x);
+    if (per <= 1) sort_batch<K, 1>(src, size, s, n, pad);
+    else if (per == 2) sort_batch<K, 2>(src, size, s, n, pad);
+    else if (per == 4) sort_batch<K, 4>(src, size, s, n, pad);
+    else if (per == 8) sort_batch<K, 8>(src, size, s, n, pad);
+    else {
+        for (int i = static_cast<int>(threadIdx.x); i < n; i += static_cast<int>(blockDim.x)) s[i] = i < size ? src[i] : pad;
+        __syncthreads();
+        bitonic_sort(s, n);
+        __syncthreads();
     }
 }
 
@@ -386,6 +509,12 @@ struct Heap {
     }
     __device__ __forceinline__ void merge(const K* a, const K* b, K* lo, K* hi) const {
         mergeG<1>(a, b, lo, hi, static_cast<int>(threadIdx.x));
+    }
+
+    // items[0, size) sorted into s0, padded with init_limits to a batch.
+    __device__ __forceinline__ void sortBatch(const K* items, int size, K* s0) const {
+        if constexpr (IPT > 0) detail::sort_batch<K, (IPT > 2 ? IPT / 2 : 1)>(items, size, s0, batchSize, init_limits);
+        else detail::sort_batch_rt<K>(items, size, s0, batchSize, init_limits);
     }
 
     // Records the first error (sticky).
@@ -589,10 +718,8 @@ struct Heap {
             if (tid == 0) parkTag = BU::kParkBase + (atomicAdd(&state->insTicket, 1) & BU::kTicketMask);
         }
 
-        // stage and pad with init_limits, then sort (:557-562)
-        for (int q = tid; q < B; q += blockDim.x) s0[q] = q < size ? items[q] : init_limits;
-        __syncthreads();
-        detail::bitonic_sort(s0, B);
+        // sort, padded with init_limits (:557-562)
+        sortBatch(items, size, s0);
 
         // lock the partial buffer (the counters are only changed under it) and
         // start loading it
@@ -698,15 +825,12 @@ struct Heap {
         K* s1 = s0 + batchSize;
         K* s2 = s1 + batchSize;
         Op op(this, ctl(s0));
-        const int B = batchSize;
         const int tid = threadIdx.x;
         int parkTag = 0;
         if constexpr (VARIANT == kBottomUp) {
             if (tid == 0) parkTag = BU::kParkBase + (atomicAdd(&state->insTicket, 1) & BU::kTicketMask);
         }
-        for (int q = tid; q < B; q += blockDim.x) s0[q] = items[q];
-        __syncthreads();
-        detail::bitonic_sort(s0, B);
+        sortBatch(items, batchSize, s0);
         if constexpr (VARIANT == kTopDown) insert_topdown(op, s0, s1, s2, target - 1, true);
         else insert_bottomup(op, s0, s1, s2, target - 1, parkTag, true);
     }

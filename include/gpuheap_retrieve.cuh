@@ -189,7 +189,7 @@ struct RetHeap {
             load(s.b1 + count, pbuf, ps);
             fill(s.b1 + count + ps, B - count - ps);
             __syncthreads();
-            detail::bitonic_sort(s.b1, B);
+            detail::sort_batch_rt<K>(s.b1, B, s.b1, B, initLimit);
             if (bc == 0) {
                 store(pbuf, s.b1, B);
             } else {
@@ -208,7 +208,7 @@ struct RetHeap {
         load(s.b2, pbuf + rem, rps);
         fill(s.b2 + rps, B - rps);
         __syncthreads();
-        detail::bitonic_sort(s.b1, B);
+        detail::sort_batch_rt<K>(s.b1, B, s.b1, B, initLimit);
         if (bc == 0) {  // straight into the root
             merge(s.b1, s.b2, node(0), pbuf);
             if (threadIdx.x == 0) {
@@ -379,7 +379,7 @@ struct RetHeap {
                 fill(s.b2 + (B - gap), gap);
             }
             __syncthreads();
-            detail::bitonic_sort(s.b1, B);
+            detail::sort_batch_rt<K>(s.b1, B, s.b1, B, initLimit);
             merge(s.b1, s.b2, s.b1, s.b2);
             if (threadIdx.x == 0) detail::st_relaxed(&state->partialBufferSize, B - gap);
         }
