@@ -255,6 +255,7 @@ static __global__ void k_init_state(HeapState* st, int deleteCount) {
         st->delServing = 0;
         st->build = 0;
         st->buildNext = 0;
+        st->delStop = 0;
         st->err = 0;
         st->errOp = 0;
         st->errNode = 0;
@@ -271,6 +272,7 @@ static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit
         st->outLimit = outLimit;
         st->delTicket = 0;
         st->delServing = 0;
+        st->delStop = 0;
     }
 }
 

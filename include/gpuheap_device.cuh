@@ -87,7 +87,8 @@ struct alignas(128) HeapState {
     int delServing;         // bulk deletes: the ticket whose holder may lock node 0 now
     int build;              // bulk insert: 1 when the reserved targets are filled by a heap build (k_build)
     int buildNext;          // heap build: next node to take, counting down
-    int pad2[7];
+    int delStop;            // bulk deletes: set by the block that found nothing more to take
+    int pad2[6];
     unsigned long long appStats[8];  // applications: counters (e.g. pops, expansions, relaxations)
 };
 
@@ -1071,13 +1072,23 @@ struct Heap {
     // until it is served, so that the blocks of a bulk delete take node 0 in
     // the order they asked for it.  Unlike racing on node 0's lock word, no
     // block can lose to the others for a whole phase.  Returns the ticket
-    // (passed on with delServing once node 0 is held), or -2 on a failed wait.
+    // (passed on with delServing once node 0 is held), or -2 on a failed wait
+    // and once a block has found nothing more to take (bulkStop): the queued
+    // blocks then leave at once instead of each finding it out in its turn,
+    // which took 1.5 us a block, 227 us at the end of every bulk delete.
     __device__ __forceinline__ int takeTurn() const {
+        if (detail::ld_relaxed(&state->delStop)) return -2;
         const int t = atomicAdd(&state->delTicket, 1);
         unsigned long long t0 = 0;
         for (unsigned it = 0; detail::ld_acquire(&state->delServing) != t; ++it)
-            if (!keep_waiting(t0, it, kSiteLockPartial, 0, t)) return -2;
+            if (detail::ld_relaxed(&state->delStop) || !keep_waiting(t0, it, kSiteLockPartial, 0, t)) return -2;
         return t;
+    }
+    // Thread 0, holding node 0: this bulk delete (`fair`) is over -- the heap
+    // is empty, the output full or the smallest key not below the threshold,
+    // and no delete in flight changes that.
+    __device__ __forceinline__ void bulkStop(bool fair) const {
+        if (fair) detail::st_relaxed(&state->delStop, 1);
     }
 
     // Thread 0: waits (bounded) until the reserved-insert turn reaches `target`.
@@ -1134,10 +1145,15 @@ struct Heap {
                 c->bc = bc; c->ps = ps; c->dc = dc;
                 const int want = bc > 0 ? batchSize : (PB ? ps : 0);
                 if (want == 0 || (sortOutput && dc + want > lim)) {
+                    bulkStop(fair);
                     unlock(0, 0);
                 } else if (bc == 0) {
-                    if (!check || __ldcg(node(0)) < threshold) c->w[0] = 1;
-                    else unlock(0, 0);
+                    if (!check || __ldcg(node(0)) < threshold) {
+                        c->w[0] = 1;
+                    } else {
+                        bulkStop(fair);
+                        unlock(0, 0);
+                    }
                 } else {
                     // deleteUpdate will take node bc (a leaf, usually not in
                     // L2): start pulling it in while this block waits for the root
@@ -1145,6 +1161,7 @@ struct Heap {
                     const bool ok1 = lock(1, 0, L, kSiteLockRoot);
                     c->abort = !ok1;
                     if (ok1 && check && !(__ldcg(node(1)) < threshold)) {
+                        bulkStop(fair);
                         unlock(1, 0);
                         unlock(0, 0);
                     } else if (ok1) {
@@ -1264,15 +1281,21 @@ struct Heap {
                 c->bc = bc; c->ps = ps; c->dc = dc;
                 const int want = bc > 0 ? B : (PB ? ps : 0);
                 if (want == 0 || (sortOutput && dc + want > lim)) {
+                    bulkStop(fair);
                     unlock(0, 0);
                 } else if (bc == 0) {
-                    if (!check || __ldcg(node(0)) < threshold) c->w[0] = 1;
-                    else unlock(0, 0);
+                    if (!check || __ldcg(node(0)) < threshold) {
+                        c->w[0] = 1;
+                    } else {
+                        bulkStop(fair);
+                        unlock(0, 0);
+                    }
                 } else {
                     if (bc > 1) detail::prefetch_l2(node(bc), nodeBytes());
                     const bool ok1 = lock(1, 0, BU::INUSE, kSiteLockRoot);
                     c->abort = !ok1;
                     if (ok1 && check && !(__ldcg(node(1)) < threshold)) {
+                        bulkStop(fair);
                         unlock(1, 0);
                         unlock(0, 0);
                     } else if (ok1) {
