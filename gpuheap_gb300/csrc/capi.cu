@@ -196,6 +196,11 @@ gh_status gh_heap_create(gh_heap** out, int key_kind, int variant, int partial_b
         if (cudaMalloc(&h->d.mbox, gh::impl::mbox_bytes(batch_size, kb)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
         if (cudaMemset(h->d.mbox, 0, sizeof(gh::impl::Mailbox)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
     }
+    if (batch_num >= gh::impl::drain_nodes(h->d)) {
+        h->d.drainBlocks = gh::impl::drain_blocks((static_cast<long long>(batch_num) + 1) * batch_size, kb, h->numSMs);
+        // without this memory bulk deletes go one by one
+        if (cudaMalloc(&h->d.drain, gh::impl::drain_bytes(h->d.drainBlocks)) != cudaSuccess) { cudaGetLastError(); h->d.drain = nullptr; }
+    }
     gh_status st = fill_items(h, nullptr);
     if (st != GH_OK) return fail(st);
     if (cudaDeviceSynchronize() != cudaSuccess) return fail(GH_ERR_CUDA);
@@ -212,6 +217,7 @@ gh_status gh_heap_destroy(gh_heap* h) {
     if (h->opSize) cudaFree(h->opSize);
     if (h->scratch) cudaFree(h->scratch);
     if (h->d.mbox) cudaFree(h->d.mbox);
+    if (h->d.drain) cudaFree(h->d.drain);
     if (h->stageIn) cudaFree(h->stageIn);
     if (h->stageOut) cudaFree(h->stageOut);
     for (cudaEvent_t e : h->sortEv)
@@ -281,16 +287,19 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
 namespace {
 // Bulk delete into out_dev in ascending order, stopping at max_keys, at an
 // empty heap or (threshold != NULL) at a smallest key not below *threshold.
+// known >= 0: the heap holds that many keys, all of which the call deletes.
 gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void* threshold, long long* n_out,
-                      void* stream) {
+                      void* stream, long long known = -1) {
     if (!h || max_keys < 0 || (max_keys > 0 && !out_dev)) return GH_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int lim = static_cast<int>(std::min<long long>(max_keys, INT_MAX));
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim, static_cast<int*>(h->d.drain),
+                                            h->d.drain ? gh::impl::kDrainWords : 0);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     if (max_keys > 0) {
-        const gh::impl::LaunchArgs a = args_of(h, s);
+        gh::impl::LaunchArgs a = args_of(h, s);
+        a.known = known;
         gh_status st = with_key(h, [&](auto k) {
             using K = decltype(k);
             K t{};
@@ -299,7 +308,7 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
         });
         if (st != GH_OK) return st;
     }
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX, nullptr, 0);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     if (n_out) {
@@ -393,7 +402,7 @@ gh_status gh_heap_concurrent(gh_heap* h, const void* keys_dev, long long n, int 
     if (a.grid < 2) a.grid = 2;  // one inserting and one deleting block at least
     const long long deletes = n / h->d.batchSize;
     const int lim = static_cast<int>(std::min<long long>(max_keys, INT_MAX));
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim, nullptr, 0);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     if (n > 0) {
@@ -404,7 +413,7 @@ gh_status gh_heap_concurrent(gh_heap* h, const void* keys_dev, long long n, int 
         });
         if (st != GH_OK) return st;
     }
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX, nullptr, 0);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     int dc = 0;
@@ -470,7 +479,8 @@ gh_status gh_heap_sort(gh_heap* h, const void* in_dev, long long n, void* out_de
     st = gh_heap_insert(h, in_dev, n, h->d.batchSize, stream);
     if (st != GH_OK) return st;
     long long got = 0;
-    st = gh_heap_delete(h, out_dev, n, &got, stream);
+    // without the partial buffer a short last batch is padded, and the padded batch does not fit the output
+    st = delete_bulk(h, out_dev, n, nullptr, &got, stream, h->d.pb || n % h->d.batchSize == 0 ? n : -1);
     if (st != GH_OK) return st;
     return got == n ? GH_OK : GH_ERR_STATE;
 }
@@ -523,10 +533,13 @@ gh_status gh_heap_sort_host(gh_heap* h, const void* keys_host, long long n, void
         if (st != GH_OK) return st;
     }
     // keys out: piece j is deleted on the caller's stream, then crosses on
-    // the copy stream while piece j + 1 is deleted
-    for (long long off = 0; off < n; off += piece) {
-        const long long len = std::min(piece, n - off);
-        st = delete_bulk(h, out + off * kb, len, nullptr, nullptr, stream);
+    // the copy stream while piece j + 1 is deleted; a heap that one sort
+    // empties (k_drain) goes in one piece
+    const bool whole = h->d.drain && h->d.ownerDepth < 0 && n / B >= gh::impl::drain_nodes(h->d);
+    const long long outPiece = whole ? n : piece;
+    for (long long off = 0; off < n; off += outPiece) {
+        const long long len = std::min(outPiece, n - off);
+        st = delete_bulk(h, out + off * kb, len, nullptr, nullptr, stream, whole ? n : -1);
         if (st != GH_OK) return st;
         GH_CUDA(cudaEventRecord(h->sortEv[e], s));
         GH_CUDA(cudaStreamWaitEvent(c, h->sortEv[e++], 0));

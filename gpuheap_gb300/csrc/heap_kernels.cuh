@@ -30,6 +30,8 @@ struct Desc {
     int keyBytes;
     void* mbox;  // owner-mode bulk delete: mailbox + lend buffers (null: plain deleteKernel only)
     int ownerDepth;  // owner-mode resident depth: -1 automatic, 0 off, else 2..4
+    void* drain;  // whole-heap deletes: DrainCtl and the digit counts (null: none)
+    int drainBlocks;  // blocks the counts have room for
 };
 
 // insertKernel: chunks of `chunk` keys, grid-strided over blocks.  `rest`:
@@ -265,8 +267,10 @@ static __global__ void k_init_state(HeapState* st, int deleteCount) {
     }
 }
 
-// Sets the HEAP_SORT cursor (unless deleteCount < 0) and the output limit.
-static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit) {
+// Sets the HEAP_SORT cursor (unless deleteCount < 0) and the output limit,
+// and zeroes `nwords` words of a bulk delete's control block.
+static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit, int* words, int nwords) {
+    for (int i = threadIdx.x; i < nwords; i += blockDim.x) words[i] = 0;
     if (threadIdx.x == 0) {
         if (deleteCount >= 0) st->deleteCount = deleteCount;
         st->outLimit = outLimit;

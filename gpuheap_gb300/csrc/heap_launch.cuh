@@ -5,6 +5,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
+#include "drain.cuh"
 #include "heap_kernels.cuh"
 #include "owner_delete.cuh"
 
@@ -19,6 +22,7 @@ struct LaunchArgs {
     int* opSize;
     bool autoThreads = false;  // `threads` / `grid` are the heap's automatic choice
     bool autoGrid = false;
+    long long known = -1;  // bulk deletes: the keys in the heap, where the caller knows (and wants them all)
     bool reserve = true;  // bulk inserts of full batches may reserve their targets (k_reserve)
 };
 
@@ -178,15 +182,48 @@ cudaError_t launch_insert_counted(const LaunchArgs& a, const K* keys, const unsi
     });
 }
 
+// The bulk delete of everything as one sort (k_drain); the kernel leaves the
+// heap to the delete loops when something has to stay in it.
+template <typename K>
+cudaError_t launch_drain(const LaunchArgs& a, K* out) {
+    return dispatch<K>(*a.d, a.threads, [&](auto proto) -> cudaError_t {
+        // the merge width plays no part: one instantiation per variant and partial buffer
+        using P = decltype(proto);
+        using H = Heap<K, P::kVariant, P::kHasPartialBuffer, 0>;
+        H h = view_of<H>(*a.d, 1);
+        const size_t smem = drain_smem(a.d->keyBytes);
+        const void* fn = reinterpret_cast<const void*>(k_drain<H, K>);
+        cudaError_t e = allow_smem<H>(fn, smem);
+        if (e != cudaSuccess) return e;
+        const int want = a.autoGrid || a.d->drainBlocks < a.grid ? a.d->drainBlocks : a.grid;
+        const int g = resident_grid(fn, kDrainThreads, smem, want);
+        DrainCtl* ctl = static_cast<DrainCtl*>(a.d->drain);
+        unsigned* cnt = reinterpret_cast<unsigned*>(static_cast<char*>(a.d->drain) + sizeof(DrainCtl));
+        int minNodes = drain_nodes(*a.d);
+        void* args[] = {&h, &out, &ctl, &cnt, &minNodes};
+        e = cudaLaunchCooperativeKernel(fn, dim3(g), dim3(kDrainThreads), args, smem, a.stream);
+        count_launch();
+        return e;
+    });
+}
+
 // Without a threshold, a heap with a mailbox first runs the owner-mode bulk
 // delete (k_delete_owner, 1024-thread blocks) while it has nodes below its
 // resident levels, then deleteKernel finishes; with a threshold,
 // deleteKernel alone.
 template <typename K>
 cudaError_t launch_erase(const LaunchArgs& a, K* out, const K* threshold) {
+    if (!threshold && a.d->drain && a.d->ownerDepth < 0) {
+        const int least = drain_nodes(*a.d);
+        if (a.known < 0 || a.known / a.d->batchSize >= least) {
+            const cudaError_t e = launch_drain<K>(a, out);
+            if (e != cudaSuccess || a.known >= 0) return e;
+        }
+    }
     const int R = a.d->ownerDepth < 0 ? owner_depth(a.d->batchSize, a.d->keyBytes) : a.d->ownerDepth;
     if (!threshold && a.d->mbox && R > 0 && a.grid >= 2) {
-        cudaError_t e = cudaMemsetAsync(a.d->mbox, 0, sizeof(Mailbox), a.stream);
+        // all but the counters, which an owner that engages writes
+        cudaError_t e = cudaMemsetAsync(a.d->mbox, 0, offsetof(Mailbox, stats), a.stream);
         if (e != cudaSuccess) return e;
         e = dispatch<K>(*a.d, 1024, [&](auto proto) -> cudaError_t {
             using H = decltype(proto);

@@ -54,7 +54,7 @@ cudaError_t run_sort(const gh::impl::Desc& d, const void* in, long long n, void*
     e = cudaMemsetAsync(d.status, 0, sizeof(int) * (static_cast<size_t>(d.batchNum) + 2), s);
     if (e != cudaSuccess) return e;
     gh::impl::k_init_state<<<1, 32, 0, s>>>(d.state, 0);
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(d.state, 0, static_cast<int>(n));
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(d.state, 0, static_cast<int>(n), nullptr, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const gh::impl::LaunchArgs a{&d, threads, grid, s, nullptr};

@@ -63,9 +63,9 @@ gh_status gh_heap_set_block_threads(gh_heap* h, int threads);
 /* Blocks for the bulk entry points (0 = one per SM). */
 gh_status gh_heap_set_grid(gh_heap* h, int blocks);
 /* Resident depth of the owner-mode bulk delete: -1 = automatic (the default:
- * the deepest of 2..4 whose levels fit in one block's shared memory), 0 = off
- * (the plain deleteKernel loop), 2..4 = levels 0..depth kept in the owner
- * block.  It has no counterpart in the reference.  GH_ERR_INVALID when the
+ * the deepest of 2..4 whose levels fit in one block's shared memory, and one
+ * sort for a whole heap), 0 = off (the plain deleteKernel loop), 2..4 =
+ * levels 0..depth kept in the owner block.  It has no counterpart in the reference.  GH_ERR_INVALID when the
  * heap has no owner mode (batch_size below 512) or the depth does not fit. */
 gh_status gh_heap_set_owner_depth(gh_heap* h, int depth);
 
@@ -84,7 +84,11 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
 /* deleteKernel (test/heap_test.cu:60-77): deleteRoot/deleteUpdate until the
  * heap is empty or the next deleted batch would not fit in max_keys.  Keys
  * are written in ascending order (HEAP_SORT) to out_dev[0, *n_out).  When
- * n_out is not NULL the call synchronizes the stream to read the count. */
+ * n_out is not NULL the call synchronizes the stream to read the count.  A
+ * heap that max_keys holds whole is emptied by one radix sort between its
+ * nodes and out_dev (from 4 nodes on, or 256 where the batch size has an
+ * owner mode) unless an owner depth was chosen; the nodes then all hold
+ * init_limits.  No other operation may use the heap during the call. */
 gh_status gh_heap_delete(gh_heap* h, void* out_dev, long long max_keys, long long* n_out, void* stream);
 
 /* deleteRoot(items, size, app_t_val) in a loop (artifacts/astar/BGPQ_B/
@@ -515,8 +519,8 @@ gh_status gh_sort_batch(int key_kind, const void* in_dev, int n, void* out_dev, 
 long long gh_launch_count(void);
 
 /* Counters of the last owner-mode bulk delete on this heap (gh_heap_delete
- * and gh_heap_sort run one when the heap is deep enough; it has no
- * counterpart in the reference, whose deleteKernel is the plain loop).  Up to
+ * runs one when the heap is deep enough and is not emptied by one sort, or
+ * when an owner depth was chosen; it has no counterpart in the reference, whose deleteKernel is the plain loop).  Up to
  * n of: [0] deletes made by the owner block, SM cycles of its delete loop
  * spent [1] waiting for the next last node, [2] waiting for a lent node to
  * come back, [3] waiting for room to lend, [4] planning paths, [5] merging;
