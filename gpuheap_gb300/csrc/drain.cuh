@@ -18,8 +18,14 @@
 //     in runs of consecutive addresses;
 //   * digits that all keys share (found with the first count) take no pass;
 //   * at the end the keys are in the output and the nodes hold init_limits
-//     again; node 0's lock word is held meanwhile, and a lock word that is
-//     not free when the kernel starts leaves the work to the delete loops.
+//     again.  Every lock word is held meanwhile; one that is not free when
+//     the kernel starts leaves the work to the delete loops.
+//
+// A bulk delete that takes many batches and leaves the rest sorts the same
+// way between the node array and a scratch array: the smallest keys go to
+// the output, the rest goes back in order, which is a heap (a node's parent
+// has a smaller index in both layouts) of the node count and partial-buffer
+// size that the deletes would have left.
 //
 // Measured on GB300: 2^28 u32 keys 6.7 ms (611 ms in owner mode), 2^27 u64
 // 8.1 ms, 2^20 u32 154 us (3.8 ms), 2^16 u32 100 us.  Bound by issue slots:
@@ -45,10 +51,11 @@ __host__ __device__ constexpr int drain_tile(int keyBytes) { return kDrainThread
 // Device words of one heap's drains; `cnt` (256 x blocks) follows.
 struct alignas(128) DrainCtl {
     int arrive;  // grid barrier: arrivals
-    int bad;     // bit 0: node 0's lock word was taken, bit 1: another one; then nothing is done
+    int bad;     // a lock word was taken: nothing is done
     int pad0[30];
     unsigned long long orAll, andNot;  // or of the keys, or of their complements
-    int pad1[28];
+    unsigned long long probe[4];       // DeleteProbe
+    int pad1[20];
     unsigned total[256];  // keys per digit of the current pass
 };
 constexpr int kDrainWords = 64;  // ints ahead of `total`, zero when a drain starts (k_set_output)
@@ -133,9 +140,13 @@ __device__ __forceinline__ unsigned scan256(unsigned v, unsigned* tmp) {
 
 }  // namespace dr
 
+// tmp == null: everything, if the heap has at least minNodes full nodes and
+// the output limit allows it.  Otherwise the `take` smallest of the `expect`
+// keys the heap must hold, tmp having room for them all.
 template <typename H, typename K>
-__global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h, K* out, DrainCtl* ctl, unsigned* cnt,
-                                                                             int minNodes) {
+__global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h, K* out, K* tmp, unsigned take,
+                                                                             unsigned expect, DrainCtl* ctl,
+                                                                             unsigned* cnt, int minNodes) {
     constexpr int IPT = drain_ipt(sizeof(K)), TILE = drain_tile(sizeof(K));
     extern __shared__ __align__(16) unsigned char gh_dyn_smem[];
     DrainSmem* sm = reinterpret_cast<DrainSmem*>(gh_dyn_smem);
@@ -153,10 +164,12 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
     const int bc = sm->bc, ps = sm->ps, dc = sm->dc, B = h.batchSize;
     const long long total = static_cast<long long>(bc) * B + ps;
     // the same in every block: the counters change only after the last barrier
-    if (sm->err || bc < minNodes || dc + total > sm->lim) return;
+    if (sm->err || (tmp ? total != expect : bc < minNodes || dc + total > sm->lim)) return;
     const unsigned n = static_cast<unsigned>(total);
+    if (!tmp) take = n;
     K* A = h.heapItems;
     K* O = out + dc;
+    K* T = tmp ? tmp : O;
     int target = 0;
 
     // this block's run of tiles
@@ -165,10 +178,17 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
     const unsigned t1 = static_cast<unsigned>(static_cast<unsigned long long>(tiles) * (blk + 1) / G);
     const unsigned k0 = t0 * TILE, k1 = t1 * TILE < n ? t1 * TILE : n;
 
-    // every lock word must be free, node 0's is taken
-    if (blk == 0 && tid == 0 && detail::cas_acquire(h.status, 0, H::lockedState()) != 0) atomicOr(&ctl->bad, 1);
-    for (int i = 1 + blk * kDrainThreads + tid; i <= bc; i += G * kDrainThreads)
-        if (detail::ld_acquire(h.status + i) != 0) atomicOr(&ctl->bad, 2);
+    // Take every lock word.  An operation still in flight holds one at any
+    // time (it locks the next node before it frees the last), so it makes
+    // this fail or waits until the end.  A thread stops at its first failure:
+    // the first `mine` of its words are its own.
+    const int stride = G * kDrainThreads;
+    int mine = 0;
+    for (int i = blk * kDrainThreads + tid; i <= bc; i += stride, ++mine)
+        if (detail::cas_acquire(h.status + i, 0, H::lockedState()) != 0) {
+            atomicOr(&ctl->bad, 1);
+            break;
+        }
 
     // key i of the sort is A[i < ps ? i : i + gap] before the first pass
     // (the partial buffer, then the nodes)
@@ -229,7 +249,7 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
             varies = __ldcg(&ctl->orAll) & __ldcg(&ctl->andNot);
             __syncthreads();
             if (sm->bad) {
-                if (blk == 0 && tid == 0 && (sm->bad & 1) == 0) detail::st_release(h.status, 0);
+                for (int i = blk * kDrainThreads + tid; mine > 0; i += stride, --mine) detail::st_release(h.status + i, 0);
                 return;
             }
             first = false;
@@ -260,7 +280,7 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
             if (tid < 256) off = b + __ldcg(&cnt[static_cast<size_t>(tid) * G + blk]);
         }
         // ---- scatter, tile by tile
-        K* dst = (passes & 1) ? A : O;
+        K* dst = (passes & 1) ? A : T;
 #pragma unroll 1
         for (unsigned base = k0; base < k1; base += TILE) {
             for (int q = tid; q < kDrainWarps * 256; q += kDrainThreads) (&sm->warpCnt[0][0])[q] = 0;
@@ -334,40 +354,93 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
         gap = 0;
         ++passes;
     }
-    // ---- the output takes the keys if they are in the node array; the nodes go back to init_limits
-    const bool inNodes = (passes & 1) == 0;
+    // ---- the sorted keys are in T or (an even number of passes) in the node array
     const size_t slots = static_cast<size_t>(bc + 1) * B;
-    const K fill = h.init_limits;
-    if (inNodes && passes == 0) {  // equal keys: straight from the nodes
-        for (size_t i = static_cast<size_t>(blk) * kDrainThreads + tid; i < n; i += static_cast<size_t>(G) * kDrainThreads)
-            O[i] = __ldcg(A + (i < static_cast<unsigned>(ps) ? i : i + gap0));
-        if (!dr::grid_sync(h, ctl, sm, target)) return;
-    }
-    const bool copy = inNodes && passes > 0;
+    const int left = bc - static_cast<int>(take / B);  // full nodes that stay (take is a multiple of B or everything)
+    const size_t at = static_cast<size_t>(blk) * kDrainThreads + tid, step = static_cast<size_t>(G) * kDrainThreads;
     constexpr int V = 16 / sizeof(K);
-    const bool vec = (reinterpret_cast<uintptr_t>(O) & 15) == 0;
-    const uint4 pat = detail::splat16<K>(fill);
+    const uint4 pat = detail::splat16<K>(h.init_limits);
     uint4* A4 = reinterpret_cast<uint4*>(A);
-    for (size_t q = static_cast<size_t>(blk) * kDrainThreads + tid; q < slots / V; q += static_cast<size_t>(G) * kDrainThreads) {
-        const size_t i = q * V;
-        if (copy && i < n) {
-            const uint4 x = __ldcg(A4 + q);
-            if (vec && i + V <= n) {
-                reinterpret_cast<uint4*>(O)[q] = x;
-            } else {
-                const K* xs = reinterpret_cast<const K*>(&x);
-#pragma unroll
-                for (int e = 0; e < V; ++e)
-                    if (i + e < n) O[i + e] = xs[e];
-            }
-        }
-        A4[q] = pat;
+    if (passes == 0 || (tmp && (passes & 1) == 0)) {  // equal keys, or keys that cannot move within the node array
+        for (size_t i = at; i < n; i += step) T[i] = __ldcg(src + (gap && i < static_cast<unsigned>(ps) ? i : i + gap));
+        if (!dr::grid_sync(h, ctl, sm, target)) return;
+        src = T;
     }
-    if (blk == 0 && tid == 0) {
-        detail::st_relaxed(&h.state->batchCount, 0);
-        detail::st_relaxed(&h.state->partialBufferSize, 0);
-        detail::st_relaxed(&h.state->deleteCount, dc + static_cast<int>(n));
-        detail::st_release(h.status, 0);
+    if (tmp) {
+        // the smallest `take` to the output, the rest to nodes 1.. and the partial buffer
+        for (size_t i = at; i < take; i += step) O[i] = __ldcg(T + i);
+        const size_t full = static_cast<size_t>(left) * B;
+        for (size_t i = at; i < slots; i += step) {
+            const size_t k = i < static_cast<size_t>(B) ? full + i : i - B;  // of the keys that stay
+            const bool has = i < static_cast<size_t>(B) ? i < static_cast<size_t>(take < n ? ps : 0) : k < full;
+            A[i] = has ? __ldcg(T + take + k) : h.init_limits;
+        }
+    } else {
+        const bool copy = src == A;
+        const bool vec = (reinterpret_cast<uintptr_t>(O) & 15) == 0;
+        for (size_t q = at; q < slots / V; q += step) {
+            const size_t i = q * V;
+            if (copy && i < n) {
+                const uint4 x = __ldcg(A4 + q);
+                if (vec && i + V <= n) {
+                    reinterpret_cast<uint4*>(O)[q] = x;
+                } else {
+                    const K* xs = reinterpret_cast<const K*>(&x);
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (i + e < n) O[i + e] = xs[e];
+                }
+            }
+            A4[q] = pat;
+        }
+    }
+    // the block that finishes last publishes the counters and frees the lock words
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        sm->ok = atomicAdd(&ctl->arrive, 1) + 1 == target + G;
+        if (sm->ok) {
+            detail::st_relaxed(&h.state->batchCount, left);
+            if (take == n) detail::st_relaxed(&h.state->partialBufferSize, 0);
+            detail::st_relaxed(&h.state->deleteCount, dc + static_cast<int>(take));
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (sm->ok)
+        for (int i = tid; i <= bc; i += kDrainThreads) detail::st_release(h.status + i, 0);
+}
+
+// Keys below `threshold` in the heap (a prefix of each node), counted by a
+// warp per node, and the counters a bulk delete plans with.
+struct DeleteProbe {
+    int bc, ps, err, pad;
+    unsigned long long below;
+};
+template <typename K>
+__global__ void __launch_bounds__(256) k_count_below(const K* __restrict__ items, const HeapState* st, int B, K threshold,
+                                                     DeleteProbe* probe) {
+    const int bc = st->batchCount, ps = st->partialBufferSize;
+    const int lane = threadIdx.x & 31;
+    unsigned long long sum = 0;
+    for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i <= bc; i += gridDim.x * 8) {
+        const K* nd = items + static_cast<size_t>(i) * B;
+        int lo = 0, hi = i == 0 ? ps : B;  // nd[lo - 1] < threshold <= nd[hi]
+        while (lo < hi) {
+            const int stp = (hi - lo + 31) / 32, p = lo + lane * stp;
+            const int c = __popc(__ballot_sync(0xffffffffu, p < hi && __ldcg(nd + p) < threshold));
+            if (c == 0) break;
+            const int nl = lo + (c - 1) * stp + 1;
+            hi = min(hi, lo + c * stp);
+            lo = nl;
+        }
+        sum += lo;
+    }
+    if (lane == 0 && sum) atomicAdd(&probe->below, sum);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        probe->bc = bc;
+        probe->ps = ps;
+        probe->err = st->err;
     }
 }
 

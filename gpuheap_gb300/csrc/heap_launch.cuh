@@ -14,6 +14,11 @@
 namespace gh {
 namespace impl {
 
+// How a bulk delete runs: the device chooses between one sort of the whole
+// heap and the delete loops, the loops, one sort of the whole heap, or one
+// sort that leaves the larger keys in the heap.
+enum class DeletePlan { kAuto, kLoops, kWhole, kPart };
+
 struct LaunchArgs {
     const Desc* d;
     int threads;
@@ -22,7 +27,9 @@ struct LaunchArgs {
     int* opSize;
     bool autoThreads = false;  // `threads` / `grid` are the heap's automatic choice
     bool autoGrid = false;
-    long long known = -1;  // bulk deletes: the keys in the heap, where the caller knows (and wants them all)
+    DeletePlan plan = DeletePlan::kAuto;
+    void* tmp = nullptr;  // kPart: scratch for `expect` keys, of which the `take` smallest leave
+    unsigned take = 0, expect = 0;
     bool reserve = true;  // bulk inserts of full batches may reserve their targets (k_reserve)
 };
 
@@ -30,6 +37,8 @@ template <typename K>
 cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int chunk);
 template <typename K>
 cudaError_t launch_erase(const LaunchArgs& a, K* out, const K* threshold = nullptr);
+template <typename K>
+cudaError_t launch_count_below(const LaunchArgs& a, K threshold);
 template <typename K>
 cudaError_t launch_erase_one(const LaunchArgs& a, K* out);
 template <typename K>
@@ -182,8 +191,18 @@ cudaError_t launch_insert_counted(const LaunchArgs& a, const K* keys, const unsi
     });
 }
 
-// The bulk delete of everything as one sort (k_drain); the kernel leaves the
-// heap to the delete loops when something has to stay in it.
+// DeleteProbe of the heap into its drain words (zeroed before).
+template <typename K>
+cudaError_t launch_count_below(const LaunchArgs& a, K threshold) {
+    DrainCtl* ctl = static_cast<DrainCtl*>(a.d->drain);
+    const int blocks = (a.d->batchNum + 8) / 8 < 4 * a.grid ? (a.d->batchNum + 8) / 8 : 4 * a.grid;
+    k_count_below<K><<<blocks, 256, 0, a.stream>>>(static_cast<const K*>(a.d->items), a.d->state, a.d->batchSize, threshold,
+                                                   reinterpret_cast<DeleteProbe*>(ctl->probe));
+    count_launch();
+    return cudaGetLastError();
+}
+
+// A bulk delete as one sort (k_drain).
 template <typename K>
 cudaError_t launch_drain(const LaunchArgs& a, K* out) {
     return dispatch<K>(*a.d, a.threads, [&](auto proto) -> cudaError_t {
@@ -200,7 +219,9 @@ cudaError_t launch_drain(const LaunchArgs& a, K* out) {
         DrainCtl* ctl = static_cast<DrainCtl*>(a.d->drain);
         unsigned* cnt = reinterpret_cast<unsigned*>(static_cast<char*>(a.d->drain) + sizeof(DrainCtl));
         int minNodes = drain_nodes(*a.d);
-        void* args[] = {&h, &out, &ctl, &cnt, &minNodes};
+        K* tmp = a.plan == DeletePlan::kPart ? static_cast<K*>(a.tmp) : nullptr;
+        unsigned take = a.take, expect = a.expect;
+        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes};
         e = cudaLaunchCooperativeKernel(fn, dim3(g), dim3(kDrainThreads), args, smem, a.stream);
         count_launch();
         return e;
@@ -213,12 +234,10 @@ cudaError_t launch_drain(const LaunchArgs& a, K* out) {
 // deleteKernel alone.
 template <typename K>
 cudaError_t launch_erase(const LaunchArgs& a, K* out, const K* threshold) {
-    if (!threshold && a.d->drain && a.d->ownerDepth < 0) {
-        const int least = drain_nodes(*a.d);
-        if (a.known < 0 || a.known / a.d->batchSize >= least) {
-            const cudaError_t e = launch_drain<K>(a, out);
-            if (e != cudaSuccess || a.known >= 0) return e;
-        }
+    const bool sorts = a.plan == DeletePlan::kWhole || a.plan == DeletePlan::kPart;
+    if (sorts || (a.plan == DeletePlan::kAuto && !threshold && a.d->drain && a.d->ownerDepth < 0)) {
+        const cudaError_t e = launch_drain<K>(a, out);
+        if (e != cudaSuccess || sorts) return e;
     }
     const int R = a.d->ownerDepth < 0 ? owner_depth(a.d->batchSize, a.d->keyBytes) : a.d->ownerDepth;
     if (!threshold && a.d->mbox && R > 0 && a.grid >= 2) {
@@ -310,6 +329,7 @@ void device_view(const Desc& d, void* out, size_t* bytes) {
 #define GH_INSTANTIATE_KEY(K)                                                                    \
     template cudaError_t launch_insert<K>(const LaunchArgs&, const K*, long long, int);          \
     template cudaError_t launch_erase<K>(const LaunchArgs&, K*, const K*);                       \
+    template cudaError_t launch_count_below<K>(const LaunchArgs&, K);                            \
     template cudaError_t launch_insert_counted<K>(const LaunchArgs&, const K*, const unsigned long long*, int); \
     template cudaError_t launch_erase_one<K>(const LaunchArgs&, K*);                             \
     template cudaError_t launch_retrieve<K>(const LaunchArgs&, K*, int, K*);                     \

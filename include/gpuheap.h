@@ -88,7 +88,11 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
  * heap that max_keys holds whole is emptied by one radix sort between its
  * nodes and out_dev (from 4 nodes on, or 256 where the batch size has an
  * owner mode) unless an owner depth was chosen; the nodes then all hold
- * init_limits.  No other operation may use the heap during the call. */
+ * init_limits.  With n_out, a call that takes many batches and leaves others
+ * sorts too, between the nodes and a scratch array of the heap's keys (up to
+ * 256 MiB stay with the heap, more is allocated for the call; without the
+ * memory the deletes go one by one), and the keys that stay go back in
+ * order. */
 gh_status gh_heap_delete(gh_heap* h, void* out_dev, long long max_keys, long long* n_out, void* stream);
 
 /* deleteRoot(items, size, app_t_val) in a loop (artifacts/astar/BGPQ_B/

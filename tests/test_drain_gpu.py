@@ -1,4 +1,5 @@
-"""GPU tests of the bulk delete of a whole heap as one radix sort (k_drain).
+"""GPU tests of the bulk deletes that are one radix sort (k_drain), of a whole
+heap and of its smallest keys.
 
 Bar: bit-exact.  The output is the sorted keys, and the heap is empty
 afterwards as the delete loops leave it: counters, lock words and every node
@@ -76,6 +77,61 @@ def test_whole_heap(variant, pb, key, B, ns):
                 assert np.array_equal(got[1:n + 1], np.sort(keys)), (n, kind)
                 assert got[0] == 0 and not got[n + 1:].any()
                 drained_ok(h, key, n, B)
+
+
+def taken_by(want, B, pb, limit=None, threshold=None):
+    """Keys a bulk delete takes: whole batches, then the partial buffer."""
+    n = len(want)
+    limit = n if limit is None else limit
+    got = 0
+    while n - got > 0:
+        size = B if n - got >= B else n - got
+        if got + size > limit or (threshold is not None and not int(want[got]) < threshold):
+            break
+        got += size
+    return got
+
+
+@pytest.mark.parametrize("variant", ["topdown", "bottomup"])
+@pytest.mark.parametrize("pb", [True, False])
+@pytest.mark.parametrize("key,B,n", [("u32", 128, 300 * 128), ("i32", 64, 8192 + 64 * 64), ("u64", 512, 400 * 512),
+                                     ("u32", 2048, 130 * 2048)])
+def test_part_of_the_heap(variant, pb, key, B, n):
+    """Limits and thresholds that leave keys behind: the smallest come out in
+    order, the rest is a valid heap of the right counts, which takes inserts
+    and gives up the rest in order."""
+    n += B // 2 + 1 if pb else 0
+    for kind in ("uniform", "two", "middle", "signed", "equal"):
+        if kind == "signed" and key != "i32":
+            continue
+        keys = make_keys(key, n, kind, n + len(kind))
+        want = np.sort(keys)
+        more = make_keys(key, 3 * B, "uniform", 1)
+        dt = torch.int64 if key == "u64" else torch.int32
+        for share in (0.4, 0.97, 1.0):
+            for how in ("limit", "threshold"):
+                limit = int(share * n) - (1 if share == 1.0 else 0)
+                thr = int(want[min(n - 1, int(share * n))])
+                exp = taken_by(want, B, pb, limit=limit) if how == "limit" else taken_by(want, B, pb, threshold=thr)
+                with gh.Heap(n // B + 4, B, key=key, variant=variant, partial_buffer=pb) as h:
+                    h.insert(to_dev(keys, key))
+                    out = torch.zeros(n + 1, dtype=dt, device="cuda")
+                    got = h.delete(out[1:], max_keys=limit) if how == "limit" else h.delete_below(out[1:], thr)
+                    assert got == exp, (kind, share, how)
+                    res = out.cpu().numpy().view(NP_KEY[key])
+                    assert np.array_equal(res[1:got + 1], want[:got]) and res[0] == 0 and not res[got + 1:].any()
+                    items, status, counters = h.snapshot()
+                    assert not status.any() and list(counters[:4]) == [(n - got) // B, (n - got) % B, got, 0]
+                    used = items[:(n - got) // B * B + B]
+                    assert np.all(items[len(used):] == NP_KEY[key](INIT[key])) or got in (0, n)  # or the loops' last root
+                    ok, msg = h.check_insert_heap()
+                    assert ok, msg
+                    h.insert(to_dev(more, key))
+                    ok, msg = h.check_insert_heap()
+                    assert ok, msg
+                    out = torch.zeros(n - got + 3 * B, dtype=dt, device="cuda")
+                    assert h.delete(out) == out.numel()
+                    assert np.array_equal(out.cpu().numpy().view(NP_KEY[key]), np.sort(np.concatenate([want[got:], more])))
 
 
 @pytest.mark.parametrize("grid", [1, 2, 7, 5000])
