@@ -116,35 +116,8 @@ gh_status with_key(const gh_heap* h, F&& f) {
     return cuda_fail(e);
 }
 
-gh_status fill_items(gh_heap* h, cudaStream_t s) {
-    const size_t n = static_cast<size_t>(h->d.batchNum + 1) * h->d.batchSize;
-    const int blocks = std::max(1, std::min<int>(h->numSMs * 8, static_cast<int>((n + 255) / 256)));
-    switch (h->keyKind) {
-        case GH_KEY_U32: {
-            uint32_t v; std::memcpy(&v, &h->d.initBits, 4);
-            gh::impl::k_fill<uint32_t><<<blocks, 256, 0, s>>>(static_cast<uint32_t*>(h->d.items), n, v);
-    gh::impl::count_launch();
-            break;
-        }
-        case GH_KEY_I32: {
-            int32_t v; std::memcpy(&v, &h->d.initBits, 4);
-            gh::impl::k_fill<int32_t><<<blocks, 256, 0, s>>>(static_cast<int32_t*>(h->d.items), n, v);
-    gh::impl::count_launch();
-            break;
-        }
-        default: {
-            uint64_t v = h->d.initBits;
-            gh::impl::k_fill<uint64_t><<<blocks, 256, 0, s>>>(static_cast<uint64_t*>(h->d.items), n, v);
-    gh::impl::count_launch();
-            break;
-        }
-    }
-    GH_CUDA(cudaGetLastError());
-    GH_CUDA(cudaMemsetAsync(h->d.status, 0, sizeof(int) * (static_cast<size_t>(h->d.batchNum) + 2), s));
-    gh::impl::k_init_state<<<1, 32, 0, s>>>(h->d.state, 0);
-    gh::impl::count_launch();
-    GH_CUDA(cudaGetLastError());
-    return GH_OK;
+gh_status fill_items(gh_heap* h, cudaStream_t s, int build = 0) {
+    return with_key(h, [&](auto k) { return gh::impl::launch_reset<decltype(k)>(h->d, h->numSMs, build, s); });
 }
 
 const char* kCheckText[] = {"ok",
@@ -364,6 +337,7 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
     const bool all = batches == bc && (ps == 0 || (total <= lim && below > bc * B));
     const long long take = all ? total : batches * B;
     if (take == 0) return GH_OK;
+    a->expect = static_cast<unsigned>(total);
     if (all) {
         if (bc >= gh::impl::drain_nodes(h->d)) a->plan = DeletePlan::kWhole;
         return GH_OK;
@@ -372,7 +346,6 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
     if (batches * (h->d.mbox && !threshold ? 4.0 : 6.0) > 120.0 + 8e-6 * bytes) {
         a->plan = DeletePlan::kPart;
         a->take = static_cast<unsigned>(take);
-        a->expect = static_cast<unsigned>(total);
     }
     return GH_OK;
 }
@@ -386,15 +359,13 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
     if (!h || max_keys < 0 || (max_keys > 0 && !out_dev)) return GH_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int lim = static_cast<int>(std::min<long long>(max_keys, INT_MAX));
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim, static_cast<int*>(h->d.drain),
-                                            h->d.drain ? gh::impl::kDrainWords : 0);
-    gh::impl::count_launch();
-    GH_CUDA(cudaGetLastError());
     gh::impl::LaunchArgs a = args_of(h, s);
     const bool sorts = h->d.drain && h->d.ownerDepth < 0;
     if (!sorts || (threshold && !n_out)) a.plan = DeletePlan::kLoops;
-    else if (known >= 0) a.plan = known / h->d.batchSize >= gh::impl::drain_nodes(h->d) ? DeletePlan::kWhole : DeletePlan::kLoops;
-    else if (n_out && max_keys > 0) {
+    else if (known >= 0) {
+        a.plan = known / h->d.batchSize >= gh::impl::drain_nodes(h->d) ? DeletePlan::kWhole : DeletePlan::kLoops;
+        a.expect = static_cast<unsigned>(known);
+    } else if (n_out && max_keys > 0) {
         gh_status st = plan_delete(h, &a, lim, threshold);
         if (st != GH_OK) return st;
     }
@@ -403,7 +374,16 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
         a.tmp = sort_scratch(h, static_cast<size_t>(a.expect) * h->d.keyBytes, s, &kept);
         if (!a.tmp) a.plan = DeletePlan::kLoops;
     }
+    // a sort that is known to come sets its limit, cursor and counters itself
+    a.lim = lim;
     const auto launch = [&]() -> gh_status {
+        const bool sorted = a.plan == DeletePlan::kWhole || a.plan == DeletePlan::kPart;
+        if (!sorted) {
+            a.lim = -1;
+            gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim);
+            gh::impl::count_launch();
+            GH_CUDA(cudaGetLastError());
+        }
         if (max_keys > 0) {
             gh_status st = with_key(h, [&](auto k) {
                 using K = decltype(k);
@@ -413,23 +393,28 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
             });
             if (st != GH_OK) return st;
         }
-        gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX, nullptr, 0);
-        gh::impl::count_launch();
-        return cuda_fail(cudaGetLastError());
+        if (!sorted) {
+            gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX);
+            gh::impl::count_launch();
+            GH_CUDA(cudaGetLastError());
+        }
+        return GH_OK;
     };
     gh_status st = launch();
     if (!kept) cudaFreeAsync(a.tmp, s);
     if (st != GH_OK || !n_out) return st;
     Counters c;
     GH_CUDA(read_counters(h, &c, s));
-    if (c.dc == 0 && c.err == 0 && (a.plan == DeletePlan::kWhole || a.plan == DeletePlan::kPart)) {
-        // a lock word was taken: the loops wait for it
-        a.plan = DeletePlan::kLoops;
-        gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim, nullptr, 0);
-        gh::impl::count_launch();
-        st = launch();
-        if (st != GH_OK) return st;
-        GH_CUDA(read_counters(h, &c, s));
+    if (a.plan == DeletePlan::kWhole || a.plan == DeletePlan::kPart) {
+        if (c.err == 0 && static_cast<long long>(c.bc) * h->d.batchSize + c.ps == a.expect) {
+            // a lock word was taken: the loops wait for it
+            a.plan = DeletePlan::kLoops;
+            st = launch();
+            if (st != GH_OK) return st;
+            GH_CUDA(read_counters(h, &c, s));
+        } else if (c.err) {
+            c.dc = 0;  // nothing was taken
+        }
     }
     *n_out = c.dc;
     return error_status(c.err);
@@ -516,7 +501,7 @@ gh_status gh_heap_concurrent(gh_heap* h, const void* keys_dev, long long n, int 
     if (a.grid < 2) a.grid = 2;  // one inserting and one deleting block at least
     const long long deletes = n / h->d.batchSize;
     const int lim = static_cast<int>(std::min<long long>(max_keys, INT_MAX));
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim, nullptr, 0);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     if (n > 0) {
@@ -527,7 +512,7 @@ gh_status gh_heap_concurrent(gh_heap* h, const void* keys_dev, long long n, int 
         });
         if (st != GH_OK) return st;
     }
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX, nullptr, 0);
+    gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX);
     gh::impl::count_launch();
     GH_CUDA(cudaGetLastError());
     int dc = 0;
@@ -583,14 +568,28 @@ gh_status gh_heap_retrieve(gh_heap* h, void* out_dev, int size, int* n_out, void
     return device_error(h);
 }
 
+namespace {
+// reset() and the insertion of n keys in batches; full batches are reserved
+// and marked with the reset, so the heap build follows at once.
+gh_status reset_and_insert(gh_heap* h, const void* keys_dev, long long n, cudaStream_t s) {
+    const int full = static_cast<int>(n / h->d.batchSize);
+    gh_status st = fill_items(h, s, full);
+    if (st != GH_OK || n == 0) return st;
+    gh::impl::LaunchArgs a = args_of(h, s);
+    a.prepared = full > 0;
+    return with_key(h, [&](auto k) {
+        using K = decltype(k);
+        return gh::impl::launch_insert<K>(a, static_cast<const K*>(keys_dev), n, h->d.batchSize);
+    });
+}
+}  // namespace
+
 gh_status gh_heap_sort(gh_heap* h, const void* in_dev, long long n, void* out_dev, void* stream) {
     gh::trace::Range range_("gh_heap_sort");
     if (!h || n < 0 || (n > 0 && (!in_dev || !out_dev))) return GH_ERR_INVALID;
     if (n > static_cast<long long>(h->d.batchNum) * h->d.batchSize) return GH_ERR_CAPACITY;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    gh_status st = fill_items(h, s);
-    if (st != GH_OK) return st;
-    st = gh_heap_insert(h, in_dev, n, h->d.batchSize, stream);
+    gh_status st = reset_and_insert(h, in_dev, n, s);
     if (st != GH_OK) return st;
     long long got = 0;
     st = delete_bulk(h, out_dev, n, nullptr, &got, stream, h->d.pb || n % h->d.batchSize == 0 ? n : -1);
@@ -634,15 +633,14 @@ gh_status gh_heap_sort_host(gh_heap* h, const void* keys_host, long long n, void
     // the copies start once the caller's stream is done with the staging buffers
     GH_CUDA(cudaEventRecord(h->sortEv[e], s));
     GH_CUDA(cudaStreamWaitEvent(c, h->sortEv[e++], 0));
-    gh_status st = fill_items(h, s);
-    if (st != GH_OK) return st;
+    gh_status st = GH_OK;
     // keys in: piece i crosses on the copy stream while piece i - 1 is inserted
     for (long long off = 0; off < n; off += piece) {
         const long long len = std::min(piece, n - off);
         GH_CUDA(cudaMemcpyAsync(in + off * kb, hin + off * kb, len * kb, cudaMemcpyHostToDevice, c));
         GH_CUDA(cudaEventRecord(h->sortEv[e], c));
         GH_CUDA(cudaStreamWaitEvent(s, h->sortEv[e++], 0));
-        st = gh_heap_insert(h, in + off * kb, len, B, stream);
+        st = off == 0 ? reset_and_insert(h, in, len, s) : gh_heap_insert(h, in + off * kb, len, B, stream);
         if (st != GH_OK) return st;
     }
     // keys out: piece j is deleted on the caller's stream, then crosses on
@@ -755,17 +753,16 @@ gh_status gh_heap_restore(gh_heap* h, const void* items_host, const int* counter
     if (bc < 0 || bc > h->d.batchNum || ps < 0 || ps >= h->d.batchSize || (!h->d.pb && ps != 0) || dc < 0)
         return GH_ERR_INVALID;
     static_assert(offsetof(gh::HeapState, partialBufferSize) == offsetof(gh::HeapState, batchCount) + sizeof(int) &&
-                      offsetof(gh::HeapState, deleteCount) == offsetof(gh::HeapState, batchCount) + 2 * sizeof(int),
-                  "batchCount, partialBufferSize and deleteCount are adjacent");
+                      offsetof(gh::HeapState, deleteCount) == offsetof(gh::HeapState, batchCount) + 2 * sizeof(int) &&
+                      offsetof(gh::HeapState, outLimit) == offsetof(gh::HeapState, batchCount) + 3 * sizeof(int),
+                  "batchCount, partialBufferSize, deleteCount and outLimit are adjacent");
     GH_CUDA(cudaDeviceSynchronize());
     GH_CUDA(cudaMemcpy(h->d.items, items_host, static_cast<size_t>(h->d.batchNum + 1) * h->d.batchSize * h->d.keyBytes,
                        cudaMemcpyHostToDevice));
     GH_CUDA(cudaMemset(h->d.status, 0, sizeof(int) * (static_cast<size_t>(h->d.batchNum) + 2)));
-    gh::impl::k_init_state<<<1, 32>>>(h->d.state, 0);
-    gh::impl::count_launch();
-    GH_CUDA(cudaGetLastError());
-    GH_CUDA(cudaDeviceSynchronize());
-    const int counters[3] = {bc, ps, dc};
+    GH_CUDA(cudaMemset(h->d.state, 0, sizeof(gh::HeapState)));
+    if (h->d.drain) GH_CUDA(cudaMemset(h->d.drain, 0, sizeof(gh::impl::DrainCtl)));
+    const int counters[4] = {bc, ps, dc, INT_MAX};
     GH_CUDA(cudaMemcpy(&h->d.state->batchCount, counters, sizeof(counters), cudaMemcpyHostToDevice));
     return GH_OK;
 }

@@ -66,7 +66,7 @@ constexpr int kBuildRatio = 48;
 // node-0 hand-offs would have moved it) and choose how to fill them;
 // otherwise reserve nothing and the insert kernel takes node 0 per batch as
 // the reference does.
-static __global__ void k_reserve(HeapState* st, int batchNum, long long m) {
+__device__ __forceinline__ void reserve_targets(HeapState* st, int batchNum, long long m) {
     const int bc = st->batchCount;
     const bool ok = m > 0 && st->err == 0 && st->partialBufferSize == 0 && bc + m <= batchNum;
     st->resvBase = bc;
@@ -76,6 +76,7 @@ static __global__ void k_reserve(HeapState* st, int batchNum, long long m) {
     st->buildNext = bc + static_cast<int>(ok ? m : 0);
     if (ok) st->batchCount = bc + static_cast<int>(m);
 }
+static __global__ void k_reserve(HeapState* st, int batchNum, long long m) { reserve_targets(st, batchNum, m); }
 
 // Step 2: the reserved targets' lock words take the state an insert holds
 // its target in (top-down TARGET, bottom-up INUSE), so that an insert that
@@ -83,7 +84,7 @@ static __global__ void k_reserve(HeapState* st, int batchNum, long long m) {
 // build holds (INUSE) every node whose batch it sifts: the targets and
 // their ancestors.
 template <typename H>
-__global__ void k_mark_reserved(const HeapState* st, int* status) {
+__device__ __forceinline__ void mark_targets(const HeapState* st, int* status) {
     const int base = st->resvBase, cnt = st->resvCount;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (!st->build) {
@@ -93,6 +94,17 @@ __global__ void k_mark_reserved(const HeapState* st, int* status) {
     }
     for (int i = 1 + t; i <= base + cnt; i += stride)
         if (i > base || H::hasDescendantIn(i, base + 1, base + cnt)) status[i] = H::lockedState();
+}
+template <typename H>
+__global__ void k_mark_reserved(const HeapState* st, int* status) { mark_targets<H>(st, status); }
+// Both steps by one block, for heaps of up to kReserveOne nodes (a launch
+// less, 2 us; one block marks 16 nodes a thread in about that).
+constexpr int kReserveOne = 16384;
+template <typename H>
+__global__ void __launch_bounds__(1024) k_reserve_mark(HeapState* st, int* status, int batchNum, long long m) {
+    if (threadIdx.x == 0) reserve_targets(st, batchNum, m);
+    __syncthreads();
+    mark_targets<H>(st, status);
 }
 
 // Step 3 of a heap build: nodes base + m .. 1 in descending order, each
@@ -237,27 +249,38 @@ __global__ void __launch_bounds__(1024) k_delete_one(H h, K* out, int* sizeOut) 
     if (threadIdx.x == 0) *sizeOut = size;
 }
 
+// reset() in one launch: every node to `fill` (16-byte stores), every lock
+// word to AVAIL, the counters, and a bulk delete's `nwords` control words.
+// build > 0 prepares the heap build that follows with that many batches
+// (what k_reserve and k_mark_reserved do for a heap in use): the targets
+// 1..build are reserved and held, and not filled, as the build writes them.
 template <typename K>
-__global__ void k_fill(K* p, size_t n, K v) {
+__global__ void __launch_bounds__(256) k_reset(K* items, int* status, HeapState* st, int batchNum, int batchSize, K fill,
+                                               int* words, int nwords, int build, int held) {
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
-}
-
-static __global__ void k_init_state(HeapState* st, int deleteCount) {
-    if (threadIdx.x == 0) {
-        st->batchCount = 0;
+    const uint4 pat = detail::splat16<K>(fill);
+    const size_t perNode = static_cast<size_t>(batchSize) * sizeof(K) / 16;
+    const size_t all = perNode * (static_cast<size_t>(batchNum) + 1), skip = perNode * build;
+    uint4* p = reinterpret_cast<uint4*>(items);
+    for (size_t i = t; i < all - skip; i += stride) p[i < perNode ? i : i + skip] = pat;
+    for (size_t i = t; i < static_cast<size_t>(batchNum) + 2; i += stride)
+        status[i] = i >= 1 && i <= static_cast<size_t>(build) ? held : 0;
+    if (t < static_cast<size_t>(nwords)) words[t] = 0;
+    if (t == 0) {
+        st->batchCount = build;
         st->partialBufferSize = 0;
-        st->deleteCount = deleteCount;
+        st->deleteCount = 0;
         st->outLimit = INT_MAX;
         st->insTicket = 0;
         st->resvBase = 0;
-        st->resvCount = 0;
+        st->resvCount = build;
         st->resvTurn = 0;
         st->delTicket = 0;
         st->delServing = 0;
-        st->build = 0;
-        st->buildNext = 0;
         st->delStop = 0;
+        st->build = build > 0;
+        st->buildNext = build;
         st->err = 0;
         st->errOp = 0;
         st->errNode = 0;
@@ -267,10 +290,8 @@ static __global__ void k_init_state(HeapState* st, int deleteCount) {
     }
 }
 
-// Sets the HEAP_SORT cursor (unless deleteCount < 0) and the output limit,
-// and zeroes `nwords` words of a bulk delete's control block.
-static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit, int* words, int nwords) {
-    for (int i = threadIdx.x; i < nwords; i += blockDim.x) words[i] = 0;
+// Sets the HEAP_SORT cursor (unless deleteCount < 0) and the output limit.
+static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit) {
     if (threadIdx.x == 0) {
         if (deleteCount >= 0) st->deleteCount = deleteCount;
         st->outLimit = outLimit;

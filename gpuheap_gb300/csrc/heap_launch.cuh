@@ -30,8 +30,24 @@ struct LaunchArgs {
     DeletePlan plan = DeletePlan::kAuto;
     void* tmp = nullptr;  // kPart: scratch for `expect` keys, of which the `take` smallest leave
     unsigned take = 0, expect = 0;
+    int lim = -1;         // kWhole, kPart: room in the output
+    bool prepared = false;  // bulk inserts: k_reset has reserved and marked the full batches' targets
     bool reserve = true;  // bulk inserts of full batches may reserve their targets (k_reserve)
 };
+
+// reset(), with the targets of `build` batches reserved and held if build > 0.
+template <typename K>
+cudaError_t launch_reset(const Desc& d, int numSMs, int build, cudaStream_t s) {
+    const size_t bytes = (static_cast<size_t>(d.batchNum) + 1) * d.batchSize * sizeof(K);
+    const size_t want = bytes / (16 * 256) + 1, most = static_cast<size_t>(numSMs) * 8;
+    K fill;
+    __builtin_memcpy(&fill, &d.initBits, sizeof(K));
+    k_reset<K><<<static_cast<int>(want < most ? want : most), 256, 0, s>>>(
+        static_cast<K*>(d.items), d.status, d.state, d.batchNum, d.batchSize, fill, static_cast<int*>(d.drain),
+        d.drain ? kDrainWords : 0, build, d.variant == kTopDown ? TD::INUSE : BU::INUSE);
+    count_launch();
+    return cudaGetLastError();
+}
 
 template <typename K>
 cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int chunk);
@@ -115,12 +131,19 @@ inline H view_of(const Desc& d, int sortOutput) {
 // so that several blocks share an SM and hide each other's lock and load
 // latency.  Measured on GB300: 2^28 u32, batch 2048: 5.7 ms at 512 threads,
 // 10.2 at 1024; 2^24 u64, batch 1024: 0.72 ms at 256, 0.76 at 512.
-inline int build_threads(int batchSize) { return batchSize >= 128 ? batchSize / 4 : 32; }
+// A build that is bound by the chain of sifts rather than by the SMs'
+// instructions (few nodes, and 8-byte keys up to about 8192) runs faster at
+// 4 keys a thread: 2^20 u64, batch 512: 107 us at 256 threads, 159 at 128;
+// 2^14 u32, batch 256: 48 us at 128, 56 at 64.
+inline int build_threads(int batchSize, int keyBytes, long long nodes) {
+    const int t = batchSize >= 128 ? batchSize / 4 : 32;
+    return 2 * t <= 512 && 2 * t <= 2 * batchSize && nodes <= (keyBytes == 8 ? 8192 : 512) ? 2 * t : t;
+}
 
 // The heap build of m reserved batches (and the `tail` keys after them).
 template <typename K>
 cudaError_t launch_build(const LaunchArgs& a, const K* keys, long long m, int tail) {
-    const int threads = a.autoThreads ? build_threads(a.d->batchSize) : a.threads;
+    const int threads = a.autoThreads ? build_threads(a.d->batchSize, a.d->keyBytes, m) : a.threads;
     return dispatch<K>(*a.d, threads, [&](auto proto) -> cudaError_t {
         using H = decltype(proto);
         const H h = view_of<H>(*a.d, 1);
@@ -149,20 +172,29 @@ cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int c
         const size_t smem = H::smemBytes(B);
         const long long m = (a.reserve && chunk == B) ? n / B : 0;
         if (m > 0) {
-            cudaError_t e = allow_smem<H>(reinterpret_cast<const void*>(k_insert_reserved<H, K>), smem);
+            if (!a.prepared) {
+                if (a.d->batchNum <= kReserveOne) {
+                    k_reserve_mark<H><<<1, 1024, 0, a.stream>>>(a.d->state, a.d->status, a.d->batchNum, m);
+                } else {
+                    k_reserve<<<1, 1, 0, a.stream>>>(a.d->state, a.d->batchNum, m);
+                    count_launch();
+                    const long long mb = (m + 255) / 256;
+                    k_mark_reserved<H><<<static_cast<int>(mb < 1024 ? mb : 1024), 256, 0, a.stream>>>(a.d->state, a.d->status);
+                }
+                count_launch();
+            }
+            cudaError_t e = launch_build<K>(a, keys, m, H::kHasPartialBuffer ? static_cast<int>(n - m * B) : 0);
             if (e != cudaSuccess) return e;
-            k_reserve<<<1, 1, 0, a.stream>>>(a.d->state, a.d->batchNum, m);
-            count_launch();
-            const long long mb = (m + 255) / 256;
-            k_mark_reserved<H><<<static_cast<int>(mb < 1024 ? mb : 1024), 256, 0, a.stream>>>(a.d->state, a.d->status);
-            count_launch();
-            e = launch_build<K>(a, keys, m, H::kHasPartialBuffer ? static_cast<int>(n - m * B) : 0);
-            if (e != cudaSuccess) return e;
-            const int g = resident_grid(reinterpret_cast<const void*>(k_insert_reserved<H, K>), a.threads, smem,
-                                        static_cast<int>(m < a.grid ? m : a.grid));
-            k_insert_reserved<H, K><<<g, a.threads, smem, a.stream>>>(h, keys, m);
-            count_launch();
-            e = cudaGetLastError();
+            if (a.prepared && (H::kHasPartialBuffer || n == m * B)) return cudaSuccess;
+            if (!a.prepared) {
+                e = allow_smem<H>(reinterpret_cast<const void*>(k_insert_reserved<H, K>), smem);
+                if (e != cudaSuccess) return e;
+                const int g = resident_grid(reinterpret_cast<const void*>(k_insert_reserved<H, K>), a.threads, smem,
+                                            static_cast<int>(m < a.grid ? m : a.grid));
+                k_insert_reserved<H, K><<<g, a.threads, smem, a.stream>>>(h, keys, m);
+                count_launch();
+                e = cudaGetLastError();
+            }
             if (e != cudaSuccess) return e;
         }
         const long long rest = n - m * B;
@@ -191,11 +223,13 @@ cudaError_t launch_insert_counted(const LaunchArgs& a, const K* keys, const unsi
     });
 }
 
-// DeleteProbe of the heap into its drain words (zeroed before).
+// DeleteProbe of the heap into its drain words.
 template <typename K>
 cudaError_t launch_count_below(const LaunchArgs& a, K threshold) {
     DrainCtl* ctl = static_cast<DrainCtl*>(a.d->drain);
     const int blocks = (a.d->batchNum + 8) / 8 < 4 * a.grid ? (a.d->batchNum + 8) / 8 : 4 * a.grid;
+    const cudaError_t e = cudaMemsetAsync(ctl->probe, 0, sizeof(ctl->probe), a.stream);
+    if (e != cudaSuccess) return e;
     k_count_below<K><<<blocks, 256, 0, a.stream>>>(static_cast<const K*>(a.d->items), a.d->state, a.d->batchSize, threshold,
                                                    reinterpret_cast<DeleteProbe*>(ctl->probe));
     count_launch();
@@ -221,7 +255,8 @@ cudaError_t launch_drain(const LaunchArgs& a, K* out) {
         int minNodes = drain_nodes(*a.d);
         K* tmp = a.plan == DeletePlan::kPart ? static_cast<K*>(a.tmp) : nullptr;
         unsigned take = a.take, expect = a.expect;
-        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes};
+        int lim = a.lim;
+        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes, &lim};
         e = cudaLaunchCooperativeKernel(fn, dim3(g), dim3(kDrainThreads), args, smem, a.stream);
         count_launch();
         return e;

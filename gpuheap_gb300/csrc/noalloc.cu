@@ -44,22 +44,17 @@ gh_status scratch_for_current_device(void** out) {
 template <typename K>
 cudaError_t run_sort(const gh::impl::Desc& d, const void* in, long long n, void* out, int threads, int grid,
                      cudaStream_t s) {
-    const size_t keys = static_cast<size_t>(d.batchNum + 1) * d.batchSize;
-    K lim;
-    std::memcpy(&lim, &d.initBits, sizeof(K));
+    const int full = static_cast<int>(n / d.batchSize);
     // every call starts from a clean heap: the array keeps the previous call's contents
-    gh::impl::k_fill<K><<<grid * 4, 256, 0, s>>>(static_cast<K*>(d.items), keys, lim);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = gh::impl::launch_reset<K>(d, grid, full, s);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(d.status, 0, sizeof(int) * (static_cast<size_t>(d.batchNum) + 2), s);
-    if (e != cudaSuccess) return e;
-    gh::impl::k_init_state<<<1, 32, 0, s>>>(d.state, 0);
-    gh::impl::k_set_output<<<1, 32, 0, s>>>(d.state, 0, static_cast<int>(n), nullptr, 0);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const gh::impl::LaunchArgs a{&d, threads, grid, s, nullptr};
+    gh::impl::LaunchArgs a{&d, threads, grid, s, nullptr, true, true};
+    a.prepared = full > 0;
     e = gh::impl::launch_insert<K>(a, static_cast<const K*>(in), n, d.batchSize);
     if (e != cudaSuccess) return e;
+    a.plan = d.drain && full >= gh::impl::drain_nodes(d) ? gh::impl::DeletePlan::kWhole : gh::impl::DeletePlan::kLoops;
+    if (a.plan == gh::impl::DeletePlan::kWhole) a.lim = static_cast<int>(n);
+    else gh::impl::k_set_output<<<1, 32, 0, s>>>(d.state, 0, static_cast<int>(n));
     return gh::impl::launch_erase<K>(a, static_cast<K*>(out));
 }
 
@@ -111,6 +106,13 @@ extern "C" gh_status gh_sort_noalloc(int key_kind, int variant, int partial_buff
     d.variant = variant;
     d.pb = partial_buffer ? 1 : 0;
     d.keyBytes = kb;
+    // one sort takes the keys out (k_drain) where its words fit the array too
+    const int blocks = gh::impl::drain_blocks(n, kb, sms);
+    if (align_up(need, 256) + gh::impl::drain_bytes(blocks) <= kNoAllocScratchBytes) {
+        d.drain = static_cast<unsigned char*>(base) + align_up(need, 256);
+        d.drainBlocks = blocks;
+        d.ownerDepth = -1;
+    }
     // threads as gh_heap_create's default: 16-byte merge runs per thread
     int ipt = 16 / kb, threads = 2 * batch_size / ipt;
     while (threads > 1024 && ipt < 8) { threads >>= 1; ipt <<= 1; }
