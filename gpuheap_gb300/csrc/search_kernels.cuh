@@ -290,7 +290,7 @@ __device__ bool run_astar(const H& heap, Inst* in, unsigned char* smem, int heap
     u64* emit = batch + B;
     int* ctl = reinterpret_cast<int*>(emit + SearchSmem::emitKeys(B, T));
     const int width = in->width, height = in->height;
-    const int goal = in->goal;
+    const int goal = in->goal, gx = goal % width, gy = goal / width;
     const bool eight = in->moves == 8;
     unsigned* g = in->g;
     const unsigned char* cost = in->cost;
@@ -313,38 +313,51 @@ __device__ bool run_astar(const H& heap, Inst* in, unsigned char* smem, int heap
                 const u64 key = batch[i];
                 const unsigned f = static_cast<unsigned>(key >> 32);
                 const int v = static_cast<int>(key & 0xffffffffu);
-                const unsigned best = __ldcg(inc);
-                const unsigned hv = astar_h(v, width, goal);
-                const unsigned gv = f - hv;
-                if (f < best && gv <= __ldcg(g + v)) {  // not pruned, not stale
+                const unsigned best = __ldcg(inc), gold = __ldcg(g + v);
+                const int x = v % width, y = v / width;
+                const unsigned gv = f - static_cast<unsigned>(abs(gx - x) + abs(gy - y));
+                if (f < best && gv <= gold) {  // not pruned, not stale
                     ++expanded;
-                    const int x = v % width, y = v / width;
+                    // Four moves side by side: their loads and then their
+                    // atomics are in flight together (move by move, each
+                    // waited for the last one's: 6.4 us a round of 256 cells).
+                    // moves 4: left, right, up, down, each costing the cell
+                    // entered; moves 8: the reference's model
+                    // (artifacts/astar/pq_model.cuh:126-190): the eight
+                    // neighbours in its order, open cells only, each
+                    // direction with its fixed cost 3 2 2 2 1 3 1 2
+#pragma unroll 1
+                    for (int k0 = 0; k0 < (eight ? 8 : 4); k0 += 4) {
+                        int u[4];
+                        unsigned cu[4], old[4], ng[4], nf[4];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        // moves 4: left, right, up, down, each costing the cell
-                        // entered; moves 8: the reference's model
-                        // (artifacts/astar/pq_model.cuh:126-190): the eight
-                        // neighbours in its order, open cells only, each
-                        // direction with its fixed cost 3 2 2 2 1 3 1 2
-                        if (k >= 4 && !eight) break;
-                        const int dx = eight ? (k < 3 ? k - 1 : k < 5 ? (k == 3 ? -1 : 1) : k - 6)
-                                             : (k == 0 ? -1 : k == 1 ? 1 : 0);
-                        const int dy = eight ? (k < 3 ? -1 : k < 5 ? 0 : 1) : (k == 2 ? -1 : k == 3 ? 1 : 0);
-                        const int nx = x + dx, ny = y + dy;
-                        if (nx < 0 || ny < 0 || nx >= width || ny >= height) continue;
-                        const int u = ny * width + nx;
-                        const unsigned cu = cost[u];
-                        if (cu == 0) continue;
-                        const unsigned c = eight ? (0x21312223u >> (4 * k)) & 15u : cu;
-                        const unsigned ng = gv + c;
-                        if (u == goal) {
-                            if (ng < __ldcg(g + u)) atomicMin(g + u, ng);
-                            atomicMin(inc, ng);
-                            continue;
+                        for (int j = 0; j < 4; ++j) {
+                            const int k = k0 + j;
+                            const int dx = eight ? (k < 3 ? k - 1 : k < 5 ? (k == 3 ? -1 : 1) : k - 6)
+                                                 : (k == 0 ? -1 : k == 1 ? 1 : 0);
+                            const int dy = eight ? (k < 3 ? -1 : k < 5 ? 0 : 1) : (k == 2 ? -1 : k == 3 ? 1 : 0);
+                            const int nx = x + dx, ny = y + dy;
+                            cu[j] = 0;
+                            u[j] = ny * width + nx;
+                            nf[j] = static_cast<unsigned>(abs(gx - nx) + abs(gy - ny));
+                            if (nx >= 0 && ny >= 0 && nx < width && ny < height) {
+                                cu[j] = cost[u[j]];
+                                old[j] = __ldcg(g + u[j]);
+                            }
                         }
-                        const unsigned nf = ng + astar_h(u, width, goal);
-                        if (nf >= __ldcg(inc) || ng >= __ldcg(g + u)) continue;
-                        if (ng < atomicMin(g + u, ng)) emit[atomicAdd(&ctl[1], 1)] = (static_cast<u64>(nf) << 32) | static_cast<unsigned>(u);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            ng[j] = gv + (eight ? (0x21312223u >> (4 * (k0 + j))) & 15u : cu[j]);
+                            nf[j] += ng[j];
+                            if (cu[j] != 0 && (u[j] == goal || nf[j] < best) && ng[j] < old[j]) old[j] = atomicMin(g + u[j], ng[j]);
+                            else cu[j] = 0;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (cu[j] == 0) continue;
+                            if (u[j] == goal) atomicMin(inc, ng[j]);
+                            else if (ng[j] < old[j]) emit[atomicAdd(&ctl[1], 1)] = (static_cast<u64>(nf[j]) << 32) | static_cast<unsigned>(u[j]);
+                        }
                     }
                 }
             }
@@ -504,7 +517,8 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
     u64* batch = reinterpret_cast<u64*>(smem);
     u64* emit = batch + B;
     long long* pre = reinterpret_cast<long long*>(emit + SearchSmem::emitKeys(B, T));
-    long long* wsum = pre + B + 1;
+    long long* first = pre + B + 1;  // within the knapsack's tables: 16 B + 264 bytes
+    long long* wsum = first + B;
     int* ctl = reinterpret_cast<int*>(wsum + 32);
     unsigned long long pops = 0, edges = 0, inserted = 0, waitStart = 0;
     int lastBusy = -1, batches = 0;
@@ -518,7 +532,7 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
         size = gh::app::take_batch(heap, batch, heapOff);
         pops += size;
         if (size > 0)
-            gh::app::sssp_relax_batch(heap, batch, size, pre, wsum, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
+            gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
                                       heapOff, edges, inserted);
         gh::app::batch_done(heap.state);
         if (heap.failed()) break;

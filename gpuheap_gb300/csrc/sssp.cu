@@ -65,10 +65,13 @@ __global__ void k_sssp_init(unsigned* dist, int n, int source, gh::HeapState* st
 
 // Shared memory of one block, ahead of the heap's own region.
 struct SsspSmem {
-    static __host__ __device__ size_t bytes(int B) {
+    static __host__ __device__ size_t emitKeys(int B, int T) {
+        return static_cast<size_t>(B) + gh::app::kRelaxEdges * static_cast<size_t>(T);
+    }
+    static __host__ __device__ size_t bytes(int B, int T) {
         return static_cast<size_t>(B) * 8        // batch taken from the heap
-               + 2 * static_cast<size_t>(B) * 8  // keys waiting to be inserted
-               + (static_cast<size_t>(B) + 1) * 8 // degree prefix
+               + emitKeys(B, T) * 8              // keys waiting to be inserted
+               + (2 * static_cast<size_t>(B) + 1) * 8  // degree prefix, first edges
                + 32 * 8 + 32;                     // warp sums, control words
     }
 };
@@ -83,10 +86,11 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
     const int tid = threadIdx.x;
     u64* batch = reinterpret_cast<u64*>(smem);
     u64* emit = batch + B;
-    long long* pre = reinterpret_cast<long long*>(emit + 2 * B);
-    long long* wsum = pre + B + 1;
+    long long* pre = reinterpret_cast<long long*>(emit + SsspSmem::emitKeys(B, blockDim.x));
+    long long* first = pre + B + 1;
+    long long* wsum = first + B;
     int* ctl = reinterpret_cast<int*>(wsum + 32);
-    const int heapOff = static_cast<int>(SsspSmem::bytes(B) / 4);
+    const int heapOff = static_cast<int>(SsspSmem::bytes(B, blockDim.x) / 4);
     gh::HeapState* st = heap.state;
 
     if (tid == 0) { ctl[0] = 0; ctl[1] = 0; }
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
             continue;
         }
         pops += size;
-        gh::app::sssp_relax_batch(heap, batch, size, pre, wsum, emit, &ctl[1], rowptr, col, wt, dist, heapOff, edges,
+        gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], rowptr, col, wt, dist, heapOff, edges,
                                   inserted);
         gh::app::batch_done(st);
         if (heap.failed()) break;
@@ -156,7 +160,7 @@ extern "C" gh_status gh_sssp(gh_heap* h, int n, const long long* rowptr_dev, con
     int kind = 0, variant = 0, pb = 0, bn = 0, B = 0, threads = 0, grid = 0;
     gh_status st = gh_heap_info(h, &kind, &variant, &pb, &bn, &B, &threads, &grid);
     if (st != GH_OK) return st;
-    if (kind != GH_KEY_U64 || !pb || threads > B) return GH_ERR_INVALID;  // emit buffer holds B + threads keys
+    if (kind != GH_KEY_U64 || !pb || threads > B) return GH_ERR_INVALID;
     unsigned char view[64];
     st = gh_heap_device_view(h, view, sizeof(view));
     if (st != GH_OK) return st;
@@ -167,7 +171,7 @@ extern "C" gh_status gh_sssp(gh_heap* h, int n, const long long* rowptr_dev, con
     if (st != GH_OK) return st;
     k_sssp_init<<<256, 256, 0, s>>>(dist_dev, n, source, hs);
     gh::impl::count_launch();
-    const size_t smem = SsspSmem::bytes(B) + 16 + gh::Heap<uint64_t, 0, true>::smemBytes(B);
+    const size_t smem = SsspSmem::bytes(B, threads) + 16 + gh::Heap<uint64_t, 0, true>::smemBytes(B);
     const int ipt = 2 * B / threads;
     cudaError_t e = cudaErrorInvalidValue;
     if (variant == GH_TOPDOWN) {
