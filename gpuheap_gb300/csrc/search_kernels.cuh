@@ -216,6 +216,19 @@ __device__ __forceinline__ void flush_rest(const H& heap, u64* emit, int* cnt, i
     __syncthreads();
 }
 
+// The emitted keys (`kept` of them, fewer than B) go into the heap and the
+// next batch comes out of it, in one operation.
+template <typename H>
+__device__ __forceinline__ int exchange_rest(const H& heap, u64* emit, int* cnt, int kept, u64* batch, u64 threshold,
+                                             int heapOff, unsigned long long& inserted, bool check = true) {
+    const int size = gh::app::exchange_batch(heap, emit, kept, batch, threshold, check, heapOff);
+    inserted += kept;
+    __syncthreads();
+    if (threadIdx.x == 0) *cnt = 0;
+    __syncthreads();
+    return size;
+}
+
 // Pushes the emitted keys into the ring.  One block owns the ring, so
 // nothing frees slots while it pushes: a push that would not fit sets
 // *overflow (the instance then fails with GH_ERR_CAPACITY) instead of
@@ -301,11 +314,23 @@ __device__ bool run_astar(const H& heap, Inst* in, unsigned char* smem, int heap
     __syncthreads();
     const AstarThreshold prune{inc};
     bool over = true;  // false: the batch budget ran out, the search goes on
+    int kept = 0;      // keys of the last round still to be inserted (the block stays busy)
     for (;;) {
-        if (maxBatches && batches++ == maxBatches) { over = false; break; }
-        if (gh::app::wait_for_keys(heap, &ctl[2], &in->stop, lastBusy, waitStart, prune)) break;
+        if (maxBatches && batches++ == maxBatches) {
+            over = false;
+            if (kept) {
+                flush_rest(heap, emit, &ctl[1], heapOff, inserted);
+                gh::app::batch_done(heap.state);
+            }
+            break;
+        }
         int size = 0;
-        size = gh::app::take_batch(heap, batch, prune(heap), heapOff);
+        if (kept) {
+            size = exchange_rest(heap, emit, &ctl[1], kept, batch, prune(heap), heapOff, inserted);
+        } else {
+            if (gh::app::wait_for_keys(heap, &ctl[2], &in->stop, lastBusy, waitStart, prune)) break;
+            size = gh::app::take_batch(heap, batch, prune(heap), heapOff);
+        }
         pops += size;
         for (int base = 0; base < size; base += T) {
             const int i = base + tid;
@@ -363,9 +388,9 @@ __device__ bool run_astar(const H& heap, Inst* in, unsigned char* smem, int heap
             }
             flush_full(heap, emit, &ctl[1], B, heapOff, inserted);
         }
-        flush_rest(heap, emit, &ctl[1], heapOff, inserted);
-        gh::app::batch_done(heap.state);
-        if (heap.failed()) break;
+        kept = ctl[1];  // after flush_full's barrier, or 0 with an empty batch
+        if (!kept) gh::app::batch_done(heap.state);
+        if (gh::app::halted(heap, &in->stop)) break;
     }
     if (tid == 0) {
         atomicAdd(&in->pops, pops);
@@ -404,10 +429,21 @@ __device__ bool run_knapsack(const H& heap, Inst* in, unsigned char* smem, int h
     int counter = 0, prevBest = 0;     // switch model, thread 0
     if (tid == 0) prevBest = __ldcg(best);
     bool over = true;  // false: the batch budget ran out, the search goes on
+    const bool keeps = in->order == GH_KNAP_HEAP;  // the other orders move keys between heap and ring each round
+    int kept = 0;  // keys of the last round still to be inserted (the block stays busy)
     for (;;) {
-        if (maxBatches && batches++ == maxBatches) { over = false; break; }
+        if (maxBatches && batches++ == maxBatches) {
+            over = false;
+            if (kept) {
+                flush_rest(heap, emit, &ctl[1], heapOff, inserted);
+                gh::app::batch_done(heap.state);
+            }
+            break;
+        }
         int size = 0;
-        if (mode == 0) {
+        if (kept) {
+            size = exchange_rest(heap, emit, &ctl[1], kept, batch, prune(heap), heapOff, inserted);
+        } else if (mode == 0) {
             if (gh::app::wait_for_keys(heap, &ctl[2], &in->stop, lastBusy, waitStart, prune)) break;
             size = gh::app::take_batch(heap, batch, prune(heap), heapOff);
         } else {
@@ -468,13 +504,15 @@ __device__ bool run_knapsack(const H& heap, Inst* in, unsigned char* smem, int h
             if (mode == 0) flush_full(heap, emit, &ctl[1], B, heapOff, inserted);
             else fifo_flush(fifo, emit, &ctl[1], &ctl[5], inserted);
         }
-        if (mode == 0) flush_rest(heap, emit, &ctl[1], heapOff, inserted);
+        kept = 0;
+        if (keeps) kept = ctl[1];
+        else if (mode == 0) flush_rest(heap, emit, &ctl[1], heapOff, inserted);
         else fifo_flush(fifo, emit, &ctl[1], &ctl[5], inserted);
         if (ctl[5]) {  // node pool or ring exhausted
             if (tid == 0) { in->failed = GH_ERR_CAPACITY; gh::detail::st_relaxed(&in->stop, 1); }
         }
-        if (mode == 0) gh::app::batch_done(heap.state);
-        if (heap.failed() || ctl[5] || __syncthreads_or(threadIdx.x == 0 && in->fifo != nullptr && fifo.failed())) break;
+        if (mode == 0 && !kept) gh::app::batch_done(heap.state);
+        if (gh::app::halted(heap, &in->stop) || ctl[5] || __syncthreads_or(threadIdx.x == 0 && in->fifo != nullptr && fifo.failed())) break;
         if (in->order == GH_KNAP_SWITCH) {
             // models.cuh:102-117 (FIFO) and :210-227 (heap): count batches in
             // a row that inserted children with the best profit unchanged
@@ -525,17 +563,30 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
     if (tid == 0) ctl[1] = 0;
     __syncthreads();
     bool over = true;  // false: the batch budget ran out, the search goes on
+    int kept = 0;      // keys of the last round still to be inserted (the block stays busy)
     for (;;) {
-        if (maxBatches && batches++ == maxBatches) { over = false; break; }
-        if (gh::app::wait_for_keys(heap, &ctl[2], &in->stop, lastBusy, waitStart)) break;
+        if (maxBatches && batches++ == maxBatches) {
+            over = false;
+            if (kept) {
+                flush_rest(heap, emit, &ctl[1], heapOff, inserted);
+                gh::app::batch_done(heap.state);
+            }
+            break;
+        }
         int size = 0;
-        size = gh::app::take_batch(heap, batch, heapOff);
+        if (kept) {
+            size = exchange_rest(heap, emit, &ctl[1], kept, batch, ~0ull, heapOff, inserted, false);
+        } else {
+            if (gh::app::wait_for_keys(heap, &ctl[2], &in->stop, lastBusy, waitStart)) break;
+            size = gh::app::take_batch(heap, batch, heapOff);
+        }
+        kept = 0;
         pops += size;
         if (size > 0)
-            gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
+            kept = gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
                                       heapOff, edges, inserted);
-        gh::app::batch_done(heap.state);
-        if (heap.failed()) break;
+        if (!kept) gh::app::batch_done(heap.state);
+        if (gh::app::halted(heap, &in->stop)) break;
     }
     if (tid == 0) {
         atomicAdd(&in->pops, pops);

@@ -105,19 +105,26 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
     u64 pops = 0, edges = 0, inserted = 0;
     unsigned long long waitStart = 0;
     int lastBusy = -1;
+    int kept = 0;  // keys of the last round still to be inserted (the block stays busy)
     for (;;) {
-        if (gh::app::wait_for_keys(heap, &ctl[2], nullptr, lastBusy, waitStart)) break;
-        const int size = gh::app::take_batch(heap, batch, heapOff);
-        if (size == 0) {  // another block took the last keys first
-            gh::app::batch_done(st);
-            if (heap.failed()) break;
-            continue;
+        int size;
+        if (kept) {
+            size = gh::app::exchange_batch(heap, emit, kept, batch, heap.init_limits, false, heapOff);
+            inserted += kept;
+            kept = 0;
+            __syncthreads();
+            if (tid == 0) ctl[1] = 0;
+            __syncthreads();
+        } else {
+            if (gh::app::wait_for_keys(heap, &ctl[2], nullptr, lastBusy, waitStart)) break;
+            size = gh::app::take_batch(heap, batch, heapOff);  // 0: another block took the last keys first
         }
         pops += size;
-        gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], rowptr, col, wt, dist, heapOff, edges,
-                                  inserted);
-        gh::app::batch_done(st);
-        if (heap.failed()) break;
+        if (size > 0)
+            kept = gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], rowptr, col, wt, dist,
+                                             heapOff, edges, inserted);
+        if (!kept) gh::app::batch_done(st);
+        if (gh::app::halted(heap, nullptr)) break;
     }
     if (tid == 0) {
         atomicAdd(&st->appStats[0], pops);

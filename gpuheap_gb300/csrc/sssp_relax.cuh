@@ -7,8 +7,8 @@
 // The block scans the degrees of the current keys, then relaxes the batch's
 // edges in rounds of kRelaxEdges edges per thread (a binary search over the
 // scanned degrees finds each edge's vertex), appends improved keys to `emit`
-// and inserts full batches as they form; the remainder is inserted at the
-// end.  A round is a chain of dependent loads (the search in shared memory,
+// and inserts full batches as they form; the remainder, *cnt keys, stays in
+// `emit` and its count is returned.  A round is a chain of dependent loads (the search in shared memory,
 // the edge, the distance, the atomic), so its time hardly depends on how many
 // edges a thread carries through it side by side.
 #pragma once
@@ -22,9 +22,9 @@ constexpr int kRelaxEdges = 4;
 
 // pre: batchSize + 1 long longs; first: batchSize long longs; wsum: 32 long
 // longs; emit: batchSize + kRelaxEdges * blockDim.x keys; *cnt (shared) is 0
-// on entry and on return.
+// on entry.
 template <typename H>
-__device__ __forceinline__ void sssp_relax_batch(const H& heap, const unsigned long long* batch, int size,
+__device__ __forceinline__ int sssp_relax_batch(const H& heap, const unsigned long long* batch, int size,
                                                  long long* pre, long long* first, long long* wsum,
                                                  unsigned long long* emit, int* cnt,
                                                  const long long* __restrict__ rowptr, const int* __restrict__ col,
@@ -130,12 +130,7 @@ __device__ __forceinline__ void sssp_relax_batch(const H& heap, const unsigned l
         }
         __syncthreads();
     }
-    const int rest = *cnt;
-    if (rest > 0) insert_keys(heap, emit, rest, heapOff);
-    inserted += rest;
-    __syncthreads();
-    if (tid == 0) *cnt = 0;
-    __syncthreads();
+    return *cnt;
 }
 
 }  // namespace app

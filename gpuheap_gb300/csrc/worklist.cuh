@@ -25,7 +25,21 @@ namespace app {
 // saves and restores a few of the caller's.
 template <typename H>
 __device__ __noinline__ void insert_keys(H heap, const unsigned long long* keys, int n, int heapOff) {
-    heap.insertion(reinterpret_cast<const typename H::key_type*>(keys), n, heapOff);
+    heap.insertion(reinterpret_cast<const typename H::key_type*>(keys), n, heapOff, true);
+}
+
+// Inserts keys[0, n) (0 < n <= batchSize) and takes a batch, in one hold of
+// the heap's top (Heap::exchangeMin); returns the number of keys taken.  A
+// block that comes out of a round with keys to insert goes into the next one
+// like this: it stays counted busy meanwhile, and the heap's serial part, which
+// bounds searches of several blocks, is passed once a round instead of twice.
+template <typename H>
+__device__ __noinline__ int exchange_batch(H heap, const unsigned long long* keys, int n, unsigned long long* out,
+                                           typename H::key_type threshold, bool check, int heapOff) {
+    int size = 0;
+    heap.exchangeMin(reinterpret_cast<const typename H::key_type*>(keys), n, reinterpret_cast<typename H::key_type*>(out),
+                     size, threshold, check, heapOff);
+    return size;
 }
 
 // deleteRoot with a prune threshold (keys at or above it stay); returns the
@@ -109,6 +123,14 @@ __device__ __forceinline__ bool wait_for_keys(const H& heap, int* word, const in
     __syncthreads();
     if (!r) lastBusy = -1;
     return r;
+}
+
+// Every thread calls it, block-uniform: the heap has an error or `stop` (may
+// be NULL) is set.
+template <typename H>
+__device__ __forceinline__ bool halted(const H& heap, const int* stop) {
+    return __syncthreads_or(threadIdx.x == 0 &&
+                            (detail::ld_relaxed(&heap.state->err) != 0 || (stop && detail::ld_relaxed(stop) != 0))) != 0;
 }
 
 // The block has inserted everything it generated from its batch.

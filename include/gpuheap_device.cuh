@@ -705,7 +705,14 @@ struct Heap {
     // ------------------------------------------------------------------ insertion
     // heap/tditdd/heap.cuh:536-753 (top-down) and heap/buitdd/heap.cuh:484-690
     // (bottom-up); without the partial buffer: the _np copies.
-    __device__ __forceinline__ void insertion(const K* items, int size, int smemOffset) const {
+    //
+    // `apart`: a full batch does not meet the partial buffer unless the heap
+    // has no full node.  The reference merges the two first (case 2.2); left
+    // out, node 0 is held only to draw the target, the root still ends at or
+    // below the partial buffer (an insert never raises the root's keys), and
+    // the heap holds the same keys, spread differently over its nodes.  The
+    // search kernels, whose blocks contend on node 0, insert like this.
+    __device__ __forceinline__ void insertion(const K* items, int size, int smemOffset, bool apart = false) const {
         K* s0 = region(smemOffset);
         K* s1 = s0 + batchSize;
         K* s2 = s1 + batchSize;
@@ -732,14 +739,14 @@ struct Heap {
                 c->ps = detail::ld_relaxed(&state->partialBufferSize);
                 // a full batch meeting an empty partial buffer merges with
                 // padding only: that merge (case 2.2) changes nothing, skip it
-                if (PB && !(c->ps == 0 && size == batchSize)) { op.issue(nodeBytes()); load(s1, 0, &c->bar); }
+                if (PB && !(size == batchSize && (c->ps == 0 || (apart && c->bc > 0)))) { op.issue(nodeBytes()); load(s1, 0, &c->bar); }
             }
         }
         __syncthreads();
         if (c->abort) return;
         const int bc = c->bc, ps = c->ps;
 
-        if constexpr (PB) if (!(ps == 0 && size == B)) {
+        if constexpr (PB) if (!(size == B && (ps == 0 || (apart && bc > 0)))) {
             if (!op.wait()) return;
             if (bc == 0 && size < B) {
                 if (ps == 0) {  // case 1.1 (:575-584)
@@ -1354,6 +1361,153 @@ struct Heap {
             setState(0, 0);
         }
         sift_loop(op, 1, 0, C, base + 2 * B, base + 3 * B);
+    }
+
+    // ------------------------------------------------------------------ exchangeMin
+    // insertion(items, count, smemOffset) followed by deleteMin(out, size,
+    // threshold, smemOffset), 0 < count <= batchSize, in one hold of node 0
+    // and the root: the batch meets the root directly, the smaller half is
+    // the output and the larger one joins the partial buffer (or, with it,
+    // becomes the carried batch that refills the root), so no insert walks a
+    // path and the last node is only taken when the keys do not fill a batch.
+    // What the heap holds afterwards is the same as after the two calls; how
+    // it is spread over the nodes is not.  With a smallest key not below
+    // `threshold` (check) it is the insertion alone and size is 0.
+    // Heaps with the partial buffer, views without HEAP_SORT output.
+    __device__ __forceinline__ void exchangeMin(const K* items, int count, K* out, int& size, K threshold, bool check,
+                                                int smemOffset) const {
+        static_assert(PB, "exchangeMin needs the partial buffer");
+        size = 0;
+        if (exchangeTry(items, count, out, size, threshold, check, smemOffset)) insertion(items, count, smemOffset, true);
+    }
+    // True (block-uniform): nothing done, the smallest key is not below the threshold.
+    __device__ __forceinline__ bool exchangeTry(const K* items, int count, K* out, int& size, K threshold, bool check,
+                                                int smemOffset) const {
+        K* s0 = region(smemOffset);
+        K* s1 = s0 + batchSize;
+        K* s2 = s1 + batchSize;
+        K* s3 = s2 + batchSize;
+        Op op(this, ctl(s0));
+        OpCtl* c = op.c;
+        const int B = batchSize;
+        const int tid = threadIdx.x;
+        sortBatch(items, count, s0);
+        if (tid == 0) {
+            c->w[7] = 0;
+            c->w[8] = 0;
+            bool ok = detail::ld_relaxed(&state->err) == 0 && lock(0, 0, lockedState(), kSiteLockPartial);
+            if (ok) {
+                const int bc = detail::ld_relaxed(&state->batchCount);
+                const int ps = detail::ld_relaxed(&state->partialBufferSize);
+                c->bc = bc;
+                c->ps = ps;
+                const bool last = VARIANT == kBottomUp && bc > 1 && count + ps < B;
+                if (bc > 0) {
+                    if (last) detail::prefetch_l2(node(bc), nodeBytes());
+                    ok = lock(1, 0, lockedState(), kSiteLockRoot);
+                    if (ok && last) {
+                        unsigned long long t0 = 0;
+                        int prev;
+                        for (unsigned it = 0; (prev = detail::max_acquire(status + bc, BU::INUSE)) == BU::INUSE; ++it)
+                            if (!keep_waiting(t0, it, kSiteLockLast, bc, prev)) { ok = false; break; }
+                        c->w[8] = prev;
+                    }
+                }
+                if (ok && (bc > 0 || ps > 0)) {
+                    op.issue(((bc > 0 ? 1u : 0u) + (ps > 0 ? 1u : 0u) + (last ? 1u : 0u)) * nodeBytes());
+                    if (bc > 0) load(s2, 1, &c->bar);
+                    if (ps > 0) load(s1, 0, &c->bar);
+                    if (last) load(s3, bc, &c->bar);
+                }
+            }
+            c->abort = !ok;
+        }
+        __syncthreads();
+        if (c->abort) return false;
+        const int bc = c->bc, ps = c->ps;
+        // thread 0 decides for the block: the threads' thresholds may differ
+        // (other blocks improve the incumbent meanwhile)
+        if (tid == 0) {
+            if (!op.wait0()) c->abort = 1;
+            const K mine = s0[0], theirs = bc > 0 ? s2[0] : ps > 0 ? s1[0] : mine;
+            c->w[9] = check && !((theirs < mine ? theirs : mine) < threshold);
+        }
+        __syncthreads();
+        if (c->abort) return false;
+        if (c->w[9]) {
+            // hand everything back as it was (the last node with the state it had: its content is untouched)
+            __syncthreads();
+            if (tid == 0) {
+                if (VARIANT == kBottomUp && bc > 1 && count + ps < B) unlock(bc, c->w[8]);
+                if (bc > 0) unlock(1, 0);
+                unlock(0, 0);
+            }
+            return true;
+        }
+        const int held = count + ps;  // keys outside the full nodes, before and (with the root gone) after
+        if (bc == 0) {
+            if (ps > 0) {
+                merge(s0, s1, s0, s1);
+                __syncthreads();
+            }
+            size = held < B ? held : B;
+            smem_out(out, s0, size);
+            if (held > B) store_node(0, s1);
+            else if (ps > 0) fill_node(0, ps);
+            __syncthreads();
+            if (tid == 0) {
+                detail::st_relaxed(&state->partialBufferSize, held - size);
+                unlock(0, 0);
+            }
+            return false;
+        }
+        merge(s0, s2, out, s0);  // the output, and `count` keys that stay
+        __syncthreads();
+        size = B;
+        const bool full = held >= B, last = !full && bc > 1;
+        if (VARIANT == kTopDown && last) {
+            // the last node may be handed over through the root (takeLastTopDown), whose keys are out by now
+            if (tid == 0) {
+                const bool ok = takeLastTopDown(bc, c);
+                c->abort = !ok;
+                if (ok) {
+                    op.issue(nodeBytes());
+                    load(s3, c->w[7] ? 1 : bc, &c->bar);
+                }
+            }
+            __syncthreads();
+            if (c->abort) return false;
+            if (!op.wait()) return false;
+        }
+        const int handed = c->w[7];
+        if (full) {
+            if (ps > 0) merge(s0, s1, s0, node(0));
+        } else if (last) {
+            if (ps > 0) {
+                merge(s0, s1, s1, static_cast<K*>(nullptr));
+                __syncthreads();
+                merge(s1, s3, s0, node(0));
+            } else {
+                merge(s0, s3, s0, node(0));
+            }
+            if (!handed) fill_node(bc, B);
+        } else if (ps > 0) {
+            merge(s0, s1, node(0), static_cast<K*>(nullptr));
+        } else {
+            store_node(0, s0);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            detail::st_relaxed(&state->partialBufferSize, full ? held - B : held);
+            if (!full) detail::st_relaxed(&state->batchCount, bc - 1);
+            fence();
+            if (last && !handed) setState(bc, 0);
+            if (!full && !last) setState(1, 0);
+            setState(0, 0);
+        }
+        if (!full && !last) return false;  // the root was the only full node
+        sift_loop(op, 1, 0, s0, s2, s3);
+        return false;
     }
 
     // ------------------------------------------------------------------ retrieve
