@@ -74,6 +74,7 @@ struct alignas(16) Inst {
 // keys: a full batch is inserted after every round of one key a thread, so
 // B + 8 T holds what a round adds (an A* key has up to eight neighbours).
 struct SearchSmem {
+    // (the SSSP loop's tables, 20 bytes a key, lie where the knapsack's do)
     static __host__ __device__ size_t emitKeys(int B, int T) { return static_cast<size_t>(B) + 8 * static_cast<size_t>(T); }
     static __host__ __device__ size_t bytes(int B, int T) {
         const size_t keys = (static_cast<size_t>(B) + emitKeys(B, T)) * 8;

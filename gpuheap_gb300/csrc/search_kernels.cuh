@@ -554,10 +554,8 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
     const int B = heap.batchSize, T = blockDim.x, tid = threadIdx.x;
     u64* batch = reinterpret_cast<u64*>(smem);
     u64* emit = batch + B;
-    long long* pre = reinterpret_cast<long long*>(emit + SearchSmem::emitKeys(B, T));
-    long long* first = pre + B + 1;  // within the knapsack's tables: 16 B + 264 bytes
-    long long* wsum = first + B;
-    int* ctl = reinterpret_cast<int*>(wsum + 32);
+    void* tables = emit + SearchSmem::emitKeys(B, T);  // within the knapsack's tables
+    int* ctl = reinterpret_cast<int*>(static_cast<unsigned char*>(tables) + (gh::app::relax_bytes(B) + 7) / 8 * 8);
     unsigned long long pops = 0, edges = 0, inserted = 0, waitStart = 0;
     int lastBusy = -1, batches = 0;
     if (tid == 0) ctl[1] = 0;
@@ -583,7 +581,7 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
         kept = 0;
         pops += size;
         if (size > 0)
-            kept = gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
+            kept = gh::app::sssp_relax_batch(heap, batch, size, tables, emit, &ctl[1], in->rowptr, in->col, in->wt, in->g,
                                       heapOff, edges, inserted);
         if (!kept) gh::app::batch_done(heap.state);
         if (gh::app::halted(heap, &in->stop)) break;

@@ -71,8 +71,8 @@ struct SsspSmem {
     static __host__ __device__ size_t bytes(int B, int T) {
         return static_cast<size_t>(B) * 8        // batch taken from the heap
                + emitKeys(B, T) * 8              // keys waiting to be inserted
-               + (2 * static_cast<size_t>(B) + 1) * 8  // degree prefix, first edges
-               + 32 * 8 + 32;                     // warp sums, control words
+               + (gh::app::relax_bytes(B) + 7) / 8 * 8  // the expansion's tables
+               + 32;                             // control words
     }
 };
 
@@ -86,10 +86,8 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
     const int tid = threadIdx.x;
     u64* batch = reinterpret_cast<u64*>(smem);
     u64* emit = batch + B;
-    long long* pre = reinterpret_cast<long long*>(emit + SsspSmem::emitKeys(B, blockDim.x));
-    long long* first = pre + B + 1;
-    long long* wsum = first + B;
-    int* ctl = reinterpret_cast<int*>(wsum + 32);
+    void* tables = emit + SsspSmem::emitKeys(B, blockDim.x);
+    int* ctl = reinterpret_cast<int*>(static_cast<unsigned char*>(tables) + (gh::app::relax_bytes(B) + 7) / 8 * 8);
     const int heapOff = static_cast<int>(SsspSmem::bytes(B, blockDim.x) / 4);
     gh::HeapState* st = heap.state;
 
@@ -121,7 +119,7 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
         }
         pops += size;
         if (size > 0)
-            kept = gh::app::sssp_relax_batch(heap, batch, size, pre, first, wsum, emit, &ctl[1], rowptr, col, wt, dist,
+            kept = gh::app::sssp_relax_batch(heap, batch, size, tables, emit, &ctl[1], rowptr, col, wt, dist,
                                              heapOff, edges, inserted);
         if (!kept) gh::app::batch_done(st);
         if (gh::app::halted(heap, nullptr)) break;
