@@ -1016,6 +1016,12 @@ struct Heap {
         __syncthreads();
         if (c->abort) return;
         int cur = c->w[0];
+        // one attempt at the parent, by a warp of its own while the block
+        // stores its node or thread 0 waits for a level's fence (0.4 us a level)
+        const auto tryParent = [&](int i) {
+            if (i != 1 && tid == lockThread(1)) c->w[4] = detail::cas_acquire(status + parentOf(i), BU::AVAIL, BU::INUSE) == BU::AVAIL;
+        };
+        tryParent(cur);
         store_node(cur, s0);
         __syncthreads();
         K* carried = s0;
@@ -1026,7 +1032,7 @@ struct Heap {
             if (tid == 0) {
                 bool ok = true;
                 int reload = 0;
-                if (detail::cas_acquire(status + p, BU::AVAIL, BU::INUSE) != BU::AVAIL) {
+                if (!c->w[4]) {
                     // park our node so a deleter can pass through it, then wait
                     fence();
                     setState(cur, parkTag);
@@ -1064,12 +1070,14 @@ struct Heap {
                 K* t = carried; carried = spare; spare = t;
             }
             __syncthreads();
+            if (!done) tryParent(p);
             if (tid == 0) {
                 fence();
                 setState(cur, BU::AVAIL);
                 if (done) setState(p, BU::AVAIL);
             }
             if (done) return;
+            __syncthreads();
             cur = p;
         }
         if (tid == 0) unlock(1, BU::AVAIL);  // (:685-688)
@@ -1660,8 +1668,10 @@ struct Heap {
 
     // Sift down from `cur` (held; curPrev = the state it returns to) with the
     // carried batch in C (heap/tditdd/heap.cuh:418-532, heap/buitdd/heap.cuh:
-    // 403-480).  Per level: the two lock warps take the children at once,
-    // one bulk transaction loads them, the children merge writes the larger
+    // 403-480).  Per level: two lock warps, not thread 0's, take the children
+    // at once while thread 0 still waits for the fence that releases the
+    // level above (0.9 us of a 3 us level; both go down the tree, so holding
+    // the level above a little longer closes no cycle), one bulk transaction loads them, the children merge writes the larger
     // half straight to the larger child, the case analysis against C writes
     // the current node, and one fence releases both (a second fence to free
     // the larger child before the case analysis measured slower).
@@ -1679,8 +1689,8 @@ struct Heap {
             Level lv;
             lv.l = leftOf(cur);
             lv.r = rightOrNone(lv.l);
-            if (tid == lockThread(0)) { int p = 0; c->w[3] = lv.l > limit ? kAbsent : takeChild(lv.l, p); c->w[4] = p; }
-            if (tid == lockThread(1)) { int p = 0; c->w[5] = lv.r > limit ? kAbsent : takeChild(lv.r, p); c->w[6] = p; }
+            if (tid == lockThread(1)) { int p = 0; c->w[3] = lv.l > limit ? kAbsent : takeChild(lv.l, p); c->w[4] = p; }
+            if (tid == lockThread(2)) { int p = 0; c->w[5] = lv.r > limit ? kAbsent : takeChild(lv.r, p); c->w[6] = p; }
             __syncthreads();
             if (c->w[3] < 0 || c->w[5] < 0) {
                 carried_in(cf, c);
