@@ -27,9 +27,10 @@ struct gh_heap {
     int grid;          // 0 = one block per SM
     int device;
     int numSMs;
+    void* aux;                     // one allocation: the counters, check and scratch below, the drain's words
     gh::impl::CheckResult* check;  // device scratch for gh_heap_check
-    int* opSize;                   // device word for gh_heap_delete_batch
     void* scratch;                 // one batch of keys for gh_heap_retrieve
+    gh::impl::HostWords* words;    // pinned: results of the calls that wait
     // gh_heap_sort_host: device staging buffers, a copy stream and its events
     void* stageIn = nullptr;
     void* stageOut = nullptr;
@@ -89,19 +90,8 @@ gh_status device_error(const gh_heap* h) {
     return error_status(err);
 }
 
-// The counters and the error word, after the stream's work.
-struct Counters {
-    int bc, ps, dc, lim, pad[28], err;
-};
-static_assert(offsetof(Counters, err) == offsetof(gh::HeapState, err) && offsetof(gh::HeapState, deleteCount) == 8,
-              "Counters is the head of HeapState");
-cudaError_t read_counters(const gh_heap* h, Counters* c, cudaStream_t s) {
-    const cudaError_t e = cudaMemcpyAsync(c, h->d.state, sizeof(Counters), cudaMemcpyDeviceToHost, s);
-    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
-}
-
 gh::impl::LaunchArgs args_of(const gh_heap* h, cudaStream_t s) {
-    return gh::impl::LaunchArgs{&h->d, threads_of(h), grid_of(h), s, h->opSize, h->blockThreads == 0, h->grid == 0};
+    return gh::impl::LaunchArgs{&h->d, threads_of(h), grid_of(h), s, h->words, h->blockThreads == 0, h->grid == 0};
 }
 
 // Calls f(K{}) with the heap's key type.
@@ -179,18 +169,26 @@ gh_status gh_heap_create(gh_heap** out, int key_kind, int variant, int partial_b
     const size_t itemBytes = static_cast<size_t>(batch_num + 1) * batch_size * kb;
     if (cudaMalloc(&h->d.items, itemBytes) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
     if (cudaMalloc(&h->d.status, sizeof(int) * (static_cast<size_t>(batch_num) + 2)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
-    if (cudaMalloc(&h->d.state, sizeof(gh::HeapState)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
-    if (cudaMalloc(&h->check, sizeof(gh::impl::CheckResult)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
-    if (cudaMalloc(&h->opSize, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
-    if (cudaMalloc(&h->scratch, static_cast<size_t>(batch_size) * kb) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
+    // the rest in one allocation; without room for a drain's words bulk deletes go one by one
+    const auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t checkAt = up(sizeof(gh::HeapState)), scratchAt = checkAt + up(sizeof(gh::impl::CheckResult));
+    const size_t drainAt = scratchAt + up(static_cast<size_t>(batch_size) * kb);
+    size_t drainBytes = 0;
+    if (batch_num >= gh::impl::kDrainNodes) {
+        h->d.drainBlocks = gh::impl::drain_blocks((static_cast<long long>(batch_num) + 1) * batch_size, kb, h->numSMs);
+        drainBytes = gh::impl::drain_bytes(h->d.drainBlocks);
+    }
+    if (drainBytes && cudaMalloc(&h->aux, drainAt + drainBytes) != cudaSuccess) { cudaGetLastError(); h->aux = nullptr; drainBytes = 0; }
+    if (!h->aux && cudaMalloc(&h->aux, drainAt) != cudaSuccess) { cudaGetLastError(); h->aux = nullptr; return fail(GH_ERR_CUDA); }
+    char* aux = static_cast<char*>(h->aux);
+    h->d.state = reinterpret_cast<gh::HeapState*>(aux);
+    h->check = reinterpret_cast<gh::impl::CheckResult*>(aux + checkAt);
+    h->scratch = aux + scratchAt;
+    if (drainBytes) h->d.drain = aux + drainAt;
+    if (cudaMallocHost(&h->words, sizeof(gh::impl::HostWords)) != cudaSuccess) { cudaGetLastError(); h->words = nullptr; return fail(GH_ERR_CUDA); }
     if (gh::impl::owner_depth(batch_size, kb) > 0) {
         if (cudaMalloc(&h->d.mbox, gh::impl::mbox_bytes(batch_size, kb)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
         if (cudaMemset(h->d.mbox, 0, sizeof(gh::impl::Mailbox)) != cudaSuccess) { cudaGetLastError(); return fail(GH_ERR_CUDA); }
-    }
-    if (batch_num >= gh::impl::kDrainNodes) {
-        h->d.drainBlocks = gh::impl::drain_blocks((static_cast<long long>(batch_num) + 1) * batch_size, kb, h->numSMs);
-        // without this memory bulk deletes go one by one
-        if (cudaMalloc(&h->d.drain, gh::impl::drain_bytes(h->d.drainBlocks)) != cudaSuccess) { cudaGetLastError(); h->d.drain = nullptr; }
     }
     gh_status st = fill_items(h, nullptr);
     if (st != GH_OK) return fail(st);
@@ -203,12 +201,9 @@ gh_status gh_heap_destroy(gh_heap* h) {
     if (!h) return GH_OK;
     if (h->d.items) cudaFree(h->d.items);
     if (h->d.status) cudaFree(h->d.status);
-    if (h->d.state) cudaFree(h->d.state);
-    if (h->check) cudaFree(h->check);
-    if (h->opSize) cudaFree(h->opSize);
-    if (h->scratch) cudaFree(h->scratch);
+    if (h->aux) cudaFree(h->aux);
+    if (h->words) cudaFreeHost(h->words);
     if (h->d.mbox) cudaFree(h->d.mbox);
-    if (h->d.drain) cudaFree(h->d.drain);
     if (h->stageIn) cudaFree(h->stageIn);
     if (h->stageOut) cudaFree(h->stageOut);
     if (h->sortScratch) cudaFree(h->sortScratch);
@@ -312,7 +307,6 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
     a->plan = DeletePlan::kLoops;
     const long long B = h->d.batchSize;
     long long bc, ps, below = LLONG_MAX;
-    int err;
     if (threshold) {
         gh_status st = with_key(h, [&](auto k) {
             using K = decltype(k);
@@ -321,15 +315,15 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
             return gh::impl::launch_count_below<K>(*a, t);
         });
         if (st != GH_OK) return st;
-        gh::impl::DeleteProbe p;
-        GH_CUDA(cudaMemcpyAsync(&p, static_cast<gh::impl::DrainCtl*>(h->d.drain)->probe, sizeof(p), cudaMemcpyDeviceToHost, a->stream));
-        GH_CUDA(cudaStreamSynchronize(a->stream));
-        bc = p.bc, ps = p.ps, err = p.err, below = static_cast<long long>(p.below);
     } else {
-        Counters c;
-        GH_CUDA(read_counters(h, &c, a->stream));
-        bc = c.bc, ps = c.ps, err = c.err;
+        gh::impl::k_report<<<1, 1, 0, a->stream>>>(h->d.state, h->words);
+        gh::impl::count_launch();
+        GH_CUDA(cudaGetLastError());
     }
+    GH_CUDA(cudaStreamSynchronize(a->stream));
+    bc = h->words->bc, ps = h->words->ps;
+    const int err = h->words->err;
+    if (threshold) below = static_cast<long long>(h->words->below);
     if (err) return GH_OK;
     const long long total = bc * B + ps;
     // whole batches while the smallest key left is below the threshold and the batch fits, then the partial buffer
@@ -394,30 +388,29 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
             if (st != GH_OK) return st;
         }
         if (!sorted) {
-            gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX);
+            gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, -1, INT_MAX, a.words);
             gh::impl::count_launch();
             GH_CUDA(cudaGetLastError());
         }
         return GH_OK;
     };
+    if (n_out) h->words->dc = -1;  // a sort that does not start leaves it
+    else a.words = nullptr;
     gh_status st = launch();
     if (!kept) cudaFreeAsync(a.tmp, s);
     if (st != GH_OK || !n_out) return st;
-    Counters c;
-    GH_CUDA(read_counters(h, &c, s));
-    if (a.plan == DeletePlan::kWhole || a.plan == DeletePlan::kPart) {
-        if (c.err == 0 && static_cast<long long>(c.bc) * h->d.batchSize + c.ps == a.expect) {
-            // a lock word was taken: the loops wait for it
-            a.plan = DeletePlan::kLoops;
-            st = launch();
-            if (st != GH_OK) return st;
-            GH_CUDA(read_counters(h, &c, s));
-        } else if (c.err) {
-            c.dc = 0;  // nothing was taken
-        }
+    GH_CUDA(cudaStreamSynchronize(s));
+    if (h->words->dc < 0) {  // an error, or a lock word was taken: the loops wait for it
+        *n_out = 0;
+        st = device_error(h);
+        if (st != GH_OK) return st;
+        a.plan = DeletePlan::kLoops;
+        st = launch();
+        if (st != GH_OK) return st;
+        GH_CUDA(cudaStreamSynchronize(s));
     }
-    *n_out = c.dc;
-    return error_status(c.err);
+    *n_out = h->words->dc;
+    return error_status(h->words->err);
 }
 }  // namespace
 
@@ -543,11 +536,9 @@ gh_status gh_heap_delete_batch(gh_heap* h, void* out_dev, int* size, void* strea
         return gh::impl::launch_erase_one<K>(a, static_cast<K*>(out_dev));
     });
     if (st != GH_OK) return st;
-    int sz = 0;
-    GH_CUDA(cudaMemcpyAsync(&sz, h->opSize, sizeof(int), cudaMemcpyDeviceToHost, s));
     GH_CUDA(cudaStreamSynchronize(s));
-    if (size) *size = sz;
-    return device_error(h);
+    if (size) *size = h->words->size;
+    return error_status(h->words->err);
 }
 
 gh_status gh_heap_retrieve(gh_heap* h, void* out_dev, int size, int* n_out, void* stream) {
@@ -561,11 +552,9 @@ gh_status gh_heap_retrieve(gh_heap* h, void* out_dev, int size, int* n_out, void
         return gh::impl::launch_retrieve<K>(a, static_cast<K*>(out_dev), size, static_cast<K*>(h->scratch));
     });
     if (st != GH_OK) return st;
-    int got = 0;
-    GH_CUDA(cudaMemcpyAsync(&got, h->opSize, sizeof(int), cudaMemcpyDeviceToHost, s));
     GH_CUDA(cudaStreamSynchronize(s));
-    if (n_out) *n_out = got;
-    return device_error(h);
+    if (n_out) *n_out = h->words->size;
+    return error_status(h->words->err);
 }
 
 namespace {

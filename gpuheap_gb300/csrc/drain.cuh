@@ -56,11 +56,11 @@ struct alignas(128) DrainCtl {
     int bad;     // a lock word was taken: nothing is done
     int pad0[30];
     unsigned long long orAll, andNot;  // or of the keys, or of their complements
-    unsigned long long probe[4];       // DeleteProbe
-    int pad1[20];
+    unsigned long long below;          // k_count_below
+    int pad1[26];
 };
-// Its words are zero between bulk deletes: every drain leaves them so, the
-// heap's reset after a failed wait does.
+// Its words are zero between bulk deletes: every drain and count leaves them
+// so, the heap's reset after a failed wait does.
 constexpr int kDrainWords = sizeof(DrainCtl) / sizeof(int);
 static_assert(kDrainWords == 64, "DrainCtl layout");
 
@@ -416,7 +416,8 @@ __device__ __forceinline__ int passes(const H& h, DrainCtl* ctl, unsigned* cnt, 
 template <typename H, typename K>
 __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h, K* out, K* tmp, unsigned take,
                                                                              unsigned expect, DrainCtl* ctl,
-                                                                             unsigned* cnt, int minNodes, int lim) {
+                                                                             unsigned* cnt, int minNodes, int lim,
+                                                                             HostWords* words) {
     constexpr int IPT = drain_ipt(sizeof(K)), TILE = drain_tile(sizeof(K));
     extern __shared__ __align__(16) unsigned char gh_dyn_smem[];
     DrainSmem* sm = reinterpret_cast<DrainSmem*>(gh_dyn_smem);
@@ -549,6 +550,13 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
             if (take == n) detail::st_relaxed(&h.state->partialBufferSize, 0);
             detail::st_relaxed(&h.state->deleteCount, dc + static_cast<int>(take));
             detail::st_relaxed(&h.state->outLimit, INT_MAX);
+            if (words) {
+                volatile HostWords* w = words;
+                w->err = 0;
+                w->bc = left;
+                w->ps = take == n ? 0 : ps;
+                w->dc = dc + static_cast<int>(take);
+            }
             if (!alone) dr::clear(ctl);
             H::fence();
         }
@@ -559,14 +567,10 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
 }
 
 // Keys below `threshold` in the heap (a prefix of each node), counted by a
-// warp per node, and the counters a bulk delete plans with.
-struct DeleteProbe {
-    int bc, ps, err, pad;
-    unsigned long long below;
-};
+// warp per node into *below (zero before).
 template <typename K>
 __global__ void __launch_bounds__(256) k_count_below(const K* __restrict__ items, const HeapState* st, int B, K threshold,
-                                                     DeleteProbe* probe) {
+                                                     unsigned long long* below) {
     const int bc = st->batchCount, ps = st->partialBufferSize;
     const int lane = threadIdx.x & 31;
     unsigned long long sum = 0;
@@ -583,12 +587,13 @@ __global__ void __launch_bounds__(256) k_count_below(const K* __restrict__ items
         }
         sum += lo;
     }
-    if (lane == 0 && sum) atomicAdd(&probe->below, sum);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        probe->bc = bc;
-        probe->ps = ps;
-        probe->err = st->err;
-    }
+    if (lane == 0 && sum) atomicAdd(below, sum);
+}
+// The count and the counters to the host, the count back to zero.
+static __global__ void k_report_below(const HeapState* st, unsigned long long* below, HostWords* words) {
+    static_cast<volatile HostWords*>(words)->below = *below;
+    *below = 0;
+    report(words, st, 0);
 }
 
 }  // namespace impl

@@ -34,6 +34,26 @@ struct Desc {
     int drainBlocks;  // blocks the counts have room for
 };
 
+// What a call that waits for its result reads: in pinned host memory, written
+// by the call's last kernel, so that the wait for the stream is the only
+// round trip (a copy of the result and one of the error word took 10 us more).
+struct HostWords {
+    int size;  // keys a single operation wrote
+    int err;
+    int bc, ps, dc, pad;
+    unsigned long long below;  // keys below a bulk delete's threshold
+};
+__device__ __forceinline__ void report(HostWords* w, const HeapState* st, int size) {
+    if (!w) return;
+    volatile HostWords* v = w;
+    v->size = size;
+    v->err = detail::ld_relaxed(&st->err);
+    v->bc = detail::ld_relaxed(&st->batchCount);
+    v->ps = detail::ld_relaxed(&st->partialBufferSize);
+    v->dc = detail::ld_relaxed(&st->deleteCount);
+}
+static __global__ void k_report(const HeapState* st, HostWords* w) { report(w, st, 0); }
+
 // insertKernel: chunks of `chunk` keys, grid-strided over blocks.  `rest`:
 // the keys left over by a bulk insert of full batches, which a heap build
 // has inserted already when the heap has a partial buffer.
@@ -232,21 +252,21 @@ __global__ void __launch_bounds__(1024) k_concurrent(H h, const K* __restrict__ 
     }
 }
 
-// One retrieve of up to `want` keys by one block; the count goes to *sizeOut.
+// One retrieve of up to `want` keys by one block.
 template <typename H, typename K>
-__global__ void __launch_bounds__(1024) k_retrieve(H h, K* out, int want, K* scratch, int* sizeOut) {
+__global__ void __launch_bounds__(1024) k_retrieve(H h, K* out, int want, K* scratch, HostWords* words) {
     if constexpr (H::kHasPartialBuffer) {
         int size = want;
         h.retrieve(out, size, scratch, 0);
-        if (threadIdx.x == 0) *sizeOut = size;
+        if (threadIdx.x == 0) report(words, h.state, size);
     }
 }
 
-// One delete by one block; the size goes to *sizeOut.
+// One delete by one block.
 template <typename H, typename K>
-__global__ void __launch_bounds__(1024) k_delete_one(H h, K* out, int* sizeOut) {
+__global__ void __launch_bounds__(1024) k_delete_one(H h, K* out, HostWords* words) {
     const int size = delete_root_update(h, out);
-    if (threadIdx.x == 0) *sizeOut = size;
+    if (threadIdx.x == 0) report(words, h.state, size);
 }
 
 // reset() in one launch: every node to `fill` (16-byte stores), every lock
@@ -291,13 +311,14 @@ __global__ void __launch_bounds__(256) k_reset(K* items, int* status, HeapState*
 }
 
 // Sets the HEAP_SORT cursor (unless deleteCount < 0) and the output limit.
-static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit) {
+static __global__ void k_set_output(HeapState* st, int deleteCount, int outLimit, HostWords* words = nullptr) {
     if (threadIdx.x == 0) {
         if (deleteCount >= 0) st->deleteCount = deleteCount;
         st->outLimit = outLimit;
         st->delTicket = 0;
         st->delServing = 0;
         st->delStop = 0;
+        report(words, st, 0);
     }
 }
 

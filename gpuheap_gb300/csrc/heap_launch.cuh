@@ -24,7 +24,7 @@ struct LaunchArgs {
     int threads;
     int grid;
     cudaStream_t stream;
-    int* opSize;
+    HostWords* words;  // null: nobody waits for the result
     bool autoThreads = false;  // `threads` / `grid` are the heap's automatic choice
     bool autoGrid = false;
     DeletePlan plan = DeletePlan::kAuto;
@@ -223,15 +223,15 @@ cudaError_t launch_insert_counted(const LaunchArgs& a, const K* keys, const unsi
     });
 }
 
-// DeleteProbe of the heap into its drain words.
+// The keys below `threshold` and the counters, for the host.
 template <typename K>
 cudaError_t launch_count_below(const LaunchArgs& a, K threshold) {
     DrainCtl* ctl = static_cast<DrainCtl*>(a.d->drain);
     const int blocks = (a.d->batchNum + 8) / 8 < 4 * a.grid ? (a.d->batchNum + 8) / 8 : 4 * a.grid;
-    const cudaError_t e = cudaMemsetAsync(ctl->probe, 0, sizeof(ctl->probe), a.stream);
-    if (e != cudaSuccess) return e;
     k_count_below<K><<<blocks, 256, 0, a.stream>>>(static_cast<const K*>(a.d->items), a.d->state, a.d->batchSize, threshold,
-                                                   reinterpret_cast<DeleteProbe*>(ctl->probe));
+                                                   &ctl->below);
+    count_launch();
+    k_report_below<<<1, 1, 0, a.stream>>>(a.d->state, &ctl->below, a.words);
     count_launch();
     return cudaGetLastError();
 }
@@ -256,7 +256,8 @@ cudaError_t launch_drain(const LaunchArgs& a, K* out) {
         K* tmp = a.plan == DeletePlan::kPart ? static_cast<K*>(a.tmp) : nullptr;
         unsigned take = a.take, expect = a.expect;
         int lim = a.lim;
-        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes, &lim};
+        HostWords* words = a.lim < 0 ? nullptr : a.words;
+        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes, &lim, &words};
         e = cudaLaunchCooperativeKernel(fn, dim3(g), dim3(kDrainThreads), args, smem, a.stream);
         count_launch();
         return e;
@@ -329,7 +330,7 @@ cudaError_t launch_erase_one(const LaunchArgs& a, K* out) {
         const size_t smem = H::smemBytes(a.d->batchSize);
         cudaError_t e = allow_smem<H>(reinterpret_cast<const void*>(k_delete_one<H, K>), smem);
         if (e != cudaSuccess) return e;
-        k_delete_one<H, K><<<1, a.threads, smem, a.stream>>>(h, out, a.opSize);
+        k_delete_one<H, K><<<1, a.threads, smem, a.stream>>>(h, out, a.words);
         count_launch();
         return cudaGetLastError();
     });
@@ -343,7 +344,7 @@ cudaError_t launch_retrieve(const LaunchArgs& a, K* out, int want, K* scratch) {
         const size_t smem = H::smemBytes(a.d->batchSize);
         cudaError_t e = allow_smem<H>(reinterpret_cast<const void*>(k_retrieve<H, K>), smem);
         if (e != cudaSuccess) return e;
-        k_retrieve<H, K><<<1, a.threads, smem, a.stream>>>(h, out, want, scratch, a.opSize);
+        k_retrieve<H, K><<<1, a.threads, smem, a.stream>>>(h, out, want, scratch, a.words);
         count_launch();
         return cudaGetLastError();
     });
