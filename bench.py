@@ -148,6 +148,33 @@ def algorithmic_bytes(n, B, s, pb):
     return ins, dele
 
 
+def sort_bytes(n, B, s, passes):
+    """Bytes the bulk operations of a whole heap-sort move by their design:
+    the heap build reads the keys, writes each batch and takes one sift step
+    (two nodes read, two written) per level of height of its node; the
+    one-sort delete reads the keys twice and writes them once in each of its
+    `passes`, copies them out if they end in the node array, and writes the
+    nodes back to the padding key."""
+    M = n // B
+    heights, level = 0, M
+    while level > 1:  # nodes with at least one more level below them, level by level
+        level >>= 1
+        heights += level
+    ins = s * (2 * n + 4 * B * heights)
+    dele = s * n * (3 * passes + (2 if passes % 2 == 0 else 0) + 1)
+    return ins, dele
+
+
+def varying_digits(keys):
+    """8-bit digits in which the keys (a tensor of their bits) differ."""
+    bits = keys.element_size() * 8
+    got = 0
+    for shift in range(0, bits, 8):
+        d = (keys >> shift) & 255
+        got += int(d.min()) != int(d.max())
+    return got
+
+
 def peaks():
     try:
         with open(os.path.join(REPO, "MEASURED_PEAKS.json")) as f:
@@ -392,8 +419,8 @@ def our_arm(args):
     t_del = [e[2].elapsed_time(e[3]) for e in evs]
     total_ms = max_over_ranks(total_ms, dist, "cuda")
 
-    # the owner's counters of the last timed step's bulk delete (the e2e
-    # steps below delete in pieces and would leave a piece's counters)
+    # the owner's counters of the last timed step's bulk delete, where it ran
+    # in owner mode (--owner-depth; the automatic choice sorts a whole heap)
     owner = owner_summary(h.owner_stats(), clk.summary().get("sm_mhz"))
 
     # correctness of the last step: the deleted stream is the input in key order
@@ -428,14 +455,23 @@ def our_arm(args):
         e2e = {"value": round(job_rate(n, ws, args.steps, e2e_ms), 3), "unit": "M keys/s",
                "h2d_bytes_per_step": n * s, "d2h_bytes_per_step": n * s,
                "ms_per_step": round(e2e_ms / args.steps, 3),
-               "path": "pinned host keys -> gh_heap_sort_host (8 pieces each way, copies overlapped with the "
-                       "inserts and deletes) -> pinned host output"}
+               "path": "pinned host keys -> gh_heap_sort_host (8 pieces in, copies overlapped with the inserts; 8 pieces "
+                       "out, or one after the sort of a whole heap) -> pinned host output"}
 
     value = job_rate(n, ws, args.steps, total_ms)
     ins_b, del_b = algorithmic_bytes(n, B, s, pb)
     ti, td = statistics.mean(t_ins), statistics.mean(t_del)
+    note = ("achieved = closed-form BGPQ node bytes of the phase / its CUDA-event time (for deletes: the owner-mode "
+            "launch plus the plain k_delete for the last few nodes)")
     del_kern = "k_delete_owner" if owner else "k_delete"  # the owner launch does all but the last few deletes
-    ins_kern = "k_insert_reserved"  # full batches (chunk = batch_size) into reserved targets
+    ins_kern = "k_build"  # full batches (chunk = batch_size) into an empty heap
+    sorts = args.owner_depth == -1 and n // B >= (256 if B >= 512 else 4)
+    if sorts:
+        ins_b, del_b = sort_bytes(n, B, s, varying_digits(keys))
+        del_kern = "k_drain"
+        note = ("achieved = bytes the phase's kernel moves by its design (heap build: keys, batches and one sift step a "
+                "level of height; delete: three a key and pass of its radix sort, the copy out and the reset) / its "
+                "CUDA-event time")
     kern, kb, kt = (del_kern, del_b, td) if td >= ti else (ins_kern, ins_b, ti)
     peak, peak_kind = peaks()
     achieved = kb / (kt / 1e3) / 1e9
@@ -443,9 +479,8 @@ def our_arm(args):
             "frac": round(achieved / peak, 5), "traffic": ncu_traffic(kern, args, pb),
             "kernel": kern, "peak_source": f"{peak_kind} hbm_gbs",
             "algorithmic_bytes": kb, "launch_ms": round(kt, 3),
-            "note": "achieved = closed-form BGPQ node bytes of the phase / its CUDA-event time (for deletes: the "
-                    "owner-mode launch plus the plain k_delete for the last few nodes); frac of measured; traffic = ncu "
-                    "DRAM read+write bytes of one launch of this kernel on this workload (1 pass), null if not captured"}
+            "note": note + "; frac of measured; traffic = ncu DRAM read+write bytes of one launch of this kernel on this "
+                           "workload (1 pass), null if not captured"}
     line = {
         "metric": METRIC.format(log2n=args.log2n, key=args.key), "value": round(value, 3), "unit": "M keys/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(total_ms / args.steps, 3), "higher_is_better": True,
