@@ -66,7 +66,8 @@ static bool run(int B, int threads, int blocks, bool check, unsigned seed) {
     const size_t smem = gh_heap_smem_bytes(GH_KEY_U64, B);
     cudaFuncSetAttribute(mix<gh::Heap<uint64_t, V, true, 4>>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     mix<<<blocks, threads, smem>>>(heap, dk, dops, dat, n, dout, dsizes, threshold, check);
-    bool ok = gh_heap_sync(h, nullptr) == GH_OK;
+    const gh_status st = gh_heap_sync(h, nullptr);
+    bool ok = st == GH_OK;
     std::vector<uint64_t> out(static_cast<size_t>(n) * B), rest(keys.size() + B);
     std::vector<int> sizes(n);
     cudaMemcpy(out.data(), dout, out.size() * 8, cudaMemcpyDeviceToHost);
@@ -100,8 +101,9 @@ static bool run(int B, int threads, int blocks, bool check, unsigned seed) {
     std::sort(all.begin(), all.end());
     std::sort(keys.begin(), keys.end());
     ok = ok && all == keys;
-    if (!ok) std::printf("variant %d B %d threads %d blocks %d check %d seed %u: %s %s\n", V, B, threads, blocks, check, seed, msg,
-                         cudaGetErrorString(cudaGetLastError()));
+    if (!ok)
+        std::printf("variant %d B %d threads %d blocks %d check %d seed %u: %s, heap %s, %zu of %zu keys, %s\n", V, B, threads,
+                    blocks, check, seed, gh_status_string(st), msg, all.size(), keys.size(), cudaGetErrorString(cudaGetLastError()));
     cudaFree(dk); cudaFree(dout); cudaFree(dops); cudaFree(dat); cudaFree(dsizes); cudaFree(drest);
     gh_heap_destroy(h);
     return ok;
