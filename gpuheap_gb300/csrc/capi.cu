@@ -336,6 +336,7 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
         if (bc >= gh::impl::drain_nodes(h->d)) a->plan = DeletePlan::kWhole;
         return GH_OK;
     }
+    if (total > INT_MAX) return GH_OK;  // the sort counts its keys in 32 bits
     const double bytes = static_cast<double>(total) * h->d.keyBytes;
     if (batches * (h->d.mbox && !threshold ? 4.0 : 6.0) > 120.0 + 8e-6 * bytes) {
         a->plan = DeletePlan::kPart;
