@@ -465,7 +465,7 @@ def our_arm(args):
             "launch plus the plain k_delete for the last few nodes)")
     del_kern = "k_delete_owner" if owner else "k_delete"  # the owner launch does all but the last few deletes
     ins_kern = "k_build"  # full batches (chunk = batch_size) into an empty heap
-    sorts = args.owner_depth == -1 and n // B >= (256 if B >= 512 else 4)
+    sorts = args.owner_depth == -1 and n // B >= 4
     if sorts:
         ins_b, del_b = sort_bytes(n, B, s, varying_digits(keys))
         del_kern = "k_drain"

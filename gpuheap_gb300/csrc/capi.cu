@@ -107,6 +107,7 @@ gh_status with_key(const gh_heap* h, F&& f) {
 }
 
 gh_status fill_items(gh_heap* h, cudaStream_t s, int build = 0) {
+    h->d.restored = 0;
     return with_key(h, [&](auto k) { return gh::impl::launch_reset<decltype(k)>(h->d, h->numSMs, build, s); });
 }
 
@@ -752,6 +753,7 @@ gh_status gh_heap_restore(gh_heap* h, const void* items_host, const int* counter
     GH_CUDA(cudaMemset(h->d.status, 0, sizeof(int) * (static_cast<size_t>(h->d.batchNum) + 2)));
     GH_CUDA(cudaMemset(h->d.state, 0, sizeof(gh::HeapState)));
     if (h->d.drain) GH_CUDA(cudaMemset(h->d.drain, 0, sizeof(gh::impl::DrainCtl)));
+    h->d.restored = 1;
     const int counters[4] = {bc, ps, dc, INT_MAX};
     GH_CUDA(cudaMemcpy(&h->d.state->batchCount, counters, sizeof(counters), cudaMemcpyHostToDevice));
     return GH_OK;

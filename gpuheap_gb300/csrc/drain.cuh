@@ -83,13 +83,14 @@ inline int drain_blocks(long long keys, int keyBytes, int numSMs) {
 inline size_t drain_bytes(int blocks) { return sizeof(DrainCtl) + sizeof(unsigned) * 256 * static_cast<size_t>(blocks); }
 
 // Fewest full nodes a drain takes on.  A single tile takes about as long as
-// four plain deletes and their launch.  With the owner mode
-// a delete costs 4.4 us and 256 of them 1.1 ms, so the lines cross far below
-// 256 nodes (82 us for 1024 nodes of 1024 keys); up to there the owner mode
-// stays because its counters (gh_heap_owner_stats) describe such deletes.
-constexpr int kDrainNodes = 4;         // heaps without the owner mode
-constexpr int kDrainNodesOwner = 256;  // heaps with it
-inline int drain_nodes(const Desc& d) { return d.mbox ? kDrainNodesOwner : kDrainNodes; }
+// four plain deletes and their launch; 1024 nodes of 1024 keys take 82 us,
+// and the owner mode 4.4 us for each delete, so the owner mode is never the
+// faster way to empty a heap.  Up to 256 nodes it stays for a restored heap,
+// whose deletes are replayed one by one: its counters (gh_heap_owner_stats)
+// are read to see which sift steps that very heap takes.
+constexpr int kDrainNodes = 4;
+constexpr int kDrainNodesRestored = 256;
+inline int drain_nodes(const Desc& d) { return d.mbox && d.restored ? kDrainNodesRestored : kDrainNodes; }
 
 namespace dr {
 

@@ -32,6 +32,7 @@ struct Desc {
     int ownerDepth;  // owner-mode resident depth: -1 automatic, 0 off, else 2..4
     void* drain;  // whole-heap deletes: DrainCtl and the digit counts (null: none)
     int drainBlocks;  // blocks the counts have room for
+    int restored;  // the heap's content was put back by gh_heap_restore and not reset since
 };
 
 // What a call that waits for its result reads: in pinned host memory, written

@@ -48,7 +48,7 @@ def to_dev(a, key):
 
 def drained_ok(h, key, n, B):
     items, status, counters = h.snapshot()
-    if n // B < (256 if B >= 512 else 4):  # the delete loops leave the last root's keys in node 1
+    if n // B < 4:  # the delete loops leave the last root's keys in node 1
         items[B:2 * B] = NP_KEY[key](INIT[key])
     assert np.all(items == NP_KEY[key](INIT[key])) and not status.any()
     assert list(counters[:4]) == [0, 0, n, 0]
@@ -59,8 +59,8 @@ def drained_ok(h, key, n, B):
 @pytest.mark.parametrize("key,B,ns", [("u32", 16, (3 * 16, 4 * 16, 8192 - 16, 8192, 8192 + 16)),
                                       ("i32", 256, (1024, 8192, 3 * 8192 + 256, 1 << 20)),
                                       ("u64", 64, (256, 4096 - 64, 4096, 4096 + 64, 1 << 17)),
-                                      ("u32", 1024, (255 * 1024, 256 * 1024, 300 * 1024)),
-                                      ("u64", 2048, (256 * 2048,))])
+                                      ("u32", 1024, (3 * 1024, 4 * 1024, 17 * 1024, 300 * 1024)),
+                                      ("u64", 2048, (4 * 2048, 256 * 2048))])
 def test_whole_heap(variant, pb, key, B, ns):
     for n in ns:
         n += (B - 1 if n % 3 else 1) if pb else 0
@@ -202,6 +202,28 @@ def test_captured_in_a_graph():
             torch.cuda.synchronize()
             h.sync()
             assert np.array_equal(out.cpu().numpy().view(np.uint32), np.sort(keys))
+
+
+@pytest.mark.parametrize("nodes,owner", [(200, True), (256, False)])
+def test_a_small_restored_heap_is_replayed_by_the_owner(nodes, owner):
+    """gh_heap_restore: below 256 nodes the deletes go one by one (owner mode,
+    its counters), until the next reset."""
+    B, n = 1024, nodes * 1024
+    keys = pyoracle.gen("u32", nodes, "uniform", n)
+    out = torch.zeros(n, dtype=torch.int32, device="cuda")
+    with gh.Heap(512, B, key="u32") as h:
+        h.insert(to_dev(keys, "u32"))
+        h.sync()
+        items, _, counters = h.snapshot()
+        assert h.delete(out) == n and h.owner_stats()["deletes"] == 0
+        h.restore(items, counters[:3])
+        assert h.delete(out) == n
+        assert (h.owner_stats()["deletes"] > 0) == owner
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), np.sort(keys))
+        before = h.owner_stats()["deletes"]
+        h.sort(to_dev(keys, "u32"), out)
+        assert h.owner_stats()["deletes"] == before
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), np.sort(keys))
 
 
 def test_a_chosen_owner_depth_keeps_the_owner_mode():
