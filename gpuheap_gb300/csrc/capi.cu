@@ -334,7 +334,7 @@ gh_status plan_delete(gh_heap* h, gh::impl::LaunchArgs* a, long long lim, const 
     if (take == 0) return GH_OK;
     a->expect = static_cast<unsigned>(total);
     if (all) {
-        if (bc >= gh::impl::drain_nodes(h->d)) a->plan = DeletePlan::kWhole;
+        if (gh::impl::drains_whole(total, bc, gh::impl::drain_nodes(h->d))) a->plan = DeletePlan::kWhole;
         return GH_OK;
     }
     if (total > INT_MAX) return GH_OK;  // the sort counts its keys in 32 bits
@@ -359,7 +359,8 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
     const bool sorts = h->d.drain && h->d.ownerDepth < 0;
     if (!sorts || (threshold && !n_out)) a.plan = DeletePlan::kLoops;
     else if (known >= 0) {
-        a.plan = known / h->d.batchSize >= gh::impl::drain_nodes(h->d) ? DeletePlan::kWhole : DeletePlan::kLoops;
+        a.plan = gh::impl::drains_whole(known, known / h->d.batchSize, gh::impl::drain_nodes(h->d)) ? DeletePlan::kWhole
+                                                                                                    : DeletePlan::kLoops;
         a.expect = static_cast<unsigned>(known);
     } else if (n_out && max_keys > 0) {
         gh_status st = plan_delete(h, &a, lim, threshold);
@@ -637,7 +638,7 @@ gh_status gh_heap_sort_host(gh_heap* h, const void* keys_host, long long n, void
     // keys out: piece j is deleted on the caller's stream, then crosses on
     // the copy stream while piece j + 1 is deleted; a heap that one sort
     // empties (k_drain) goes in one piece
-    const bool whole = h->d.drain && h->d.ownerDepth < 0 && n / B >= gh::impl::drain_nodes(h->d);
+    const bool whole = h->d.drain && h->d.ownerDepth < 0 && gh::impl::drains_whole(n, n / B, gh::impl::drain_nodes(h->d));
     const long long outPiece = whole ? n : piece;
     for (long long off = 0; off < n; off += outPiece) {
         const long long len = std::min(outPiece, n - off);

@@ -413,12 +413,13 @@ __device__ __forceinline__ int passes(const H& h, DrainCtl* ctl, unsigned* cnt, 
 // the output limit allows it: `lim` keys from out on or, if it is negative,
 // the heap's own limit and output cursor (k_set_output).  Otherwise the `take`
 // smallest of the `expect` keys the heap must hold, tmp having room for them
-// all.
+// all.  `must`: the caller neither runs the loops after it nor looks whether
+// it started, so that giving way is recorded as the heap's error.
 template <typename H, typename K>
 __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h, K* out, K* tmp, unsigned take,
                                                                              unsigned expect, DrainCtl* ctl,
                                                                              unsigned* cnt, int minNodes, int lim,
-                                                                             HostWords* words) {
+                                                                             HostWords* words, int must) {
     constexpr int IPT = drain_ipt(sizeof(K)), TILE = drain_tile(sizeof(K));
     extern __shared__ __align__(16) unsigned char gh_dyn_smem[];
     DrainSmem* sm = reinterpret_cast<DrainSmem*>(gh_dyn_smem);
@@ -437,7 +438,11 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
     const int bc = sm->bc, ps = sm->ps, dc = sm->dc, B = h.batchSize;
     const long long total = static_cast<long long>(bc) * B + ps;
     // the same in every block: the counters change only after the last barrier
-    if (sm->err || (tmp ? total != expect : bc < minNodes || dc + total > sm->lim)) return;
+    if (sm->err) return;
+    if (tmp ? total != expect : bc < minNodes || dc + total > sm->lim) {
+        if (must && blk == 0 && tid == 0) h.raise(kErrInvalid, kSiteCapacity, bc, ps);
+        return;
+    }
     const unsigned n = static_cast<unsigned>(total);
     if (!tmp) take = n;
     K* A = h.heapItems;
@@ -464,7 +469,8 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
     const int stride = G * kDrainThreads;
     int mine = 0;
     for (int i = blk * kDrainThreads + tid; i <= bc; i += stride, ++mine)
-        if (detail::cas_acquire(h.status + i, 0, H::lockedState()) != 0) {
+        if (const int held = detail::cas_acquire(h.status + i, 0, H::lockedState()); held != 0) {
+            if (must) h.raise(kErrTimeout, kSiteLockPath, i, held);
             if (alone) sm->bad = 1;
             else atomicOr(&ctl->bad, 1);
             break;

@@ -7,17 +7,13 @@
 
 #include <cstddef>
 
+#include "delete_plan.h"
 #include "drain.cuh"
 #include "heap_kernels.cuh"
 #include "owner_delete.cuh"
 
 namespace gh {
 namespace impl {
-
-// How a bulk delete runs: the device chooses between one sort of the whole
-// heap and the delete loops, the loops, one sort of the whole heap, or one
-// sort that leaves the larger keys in the heap.
-enum class DeletePlan { kAuto, kLoops, kWhole, kPart };
 
 struct LaunchArgs {
     const Desc* d;
@@ -257,7 +253,9 @@ cudaError_t launch_drain(const LaunchArgs& a, K* out) {
         unsigned take = a.take, expect = a.expect;
         int lim = a.lim;
         HostWords* words = a.lim < 0 ? nullptr : a.words;
-        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes, &lim, &words};
+        // no loops follow and nobody reads `words`: a sort that does not start is an error of the heap
+        int must = a.lim >= 0 && !a.words;
+        void* args[] = {&h, &out, &tmp, &take, &expect, &ctl, &cnt, &minNodes, &lim, &words, &must};
         e = cudaLaunchCooperativeKernel(fn, dim3(g), dim3(kDrainThreads), args, smem, a.stream);
         count_launch();
         return e;

@@ -52,7 +52,8 @@ cudaError_t run_sort(const gh::impl::Desc& d, const void* in, long long n, void*
     a.prepared = full > 0;
     e = gh::impl::launch_insert<K>(a, static_cast<const K*>(in), n, d.batchSize);
     if (e != cudaSuccess) return e;
-    a.plan = d.drain && full >= gh::impl::drain_nodes(d) ? gh::impl::DeletePlan::kWhole : gh::impl::DeletePlan::kLoops;
+    a.plan = d.drain && gh::impl::drains_whole(n, full, gh::impl::drain_nodes(d)) ? gh::impl::DeletePlan::kWhole
+                                                                                  : gh::impl::DeletePlan::kLoops;
     if (a.plan == gh::impl::DeletePlan::kWhole) a.lim = static_cast<int>(n);
     else gh::impl::k_set_output<<<1, 32, 0, s>>>(d.state, 0, static_cast<int>(n));
     return gh::impl::launch_erase<K>(a, static_cast<K*>(out));
