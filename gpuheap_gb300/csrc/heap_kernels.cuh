@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(256) k_reset(K* items, int* status, HeapState*
         st->delTicket = 0;
         st->delServing = 0;
         st->delStop = 0;
+        st->progressNs = 0;
         st->build = build > 0;
         st->buildNext = build;
         st->err = 0;

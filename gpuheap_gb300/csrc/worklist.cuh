@@ -7,8 +7,12 @@
 // heap is empty while busy is 0: no block holds keys that could still be
 // inserted.  A block that finds the heap empty only reads busy, so waiting
 // blocks cannot keep each other alive; the block that takes a batch counts
-// itself before it can empty the heap.  The reference's applications stop on
-// a count of active blocks in the same way (applications/sssp_longfei_new/
+// itself before it can empty the heap.  A block may stay counted over many
+// rounds (exchange_batch) and may win the race for node 0 many times in a
+// row, so the blocks stamp what they finish (HeapState::progressNs): a wait
+// times out when the search stands still for the time limit, not when this
+// block does.  The reference's applications stop on a count of active blocks in
+// the same way (applications/sssp_longfei_new/
 // sssp.cu:19-132, artifacts/knapsack/models_pq.cuh:52-137 activeCount).
 #pragma once
 #include <type_traits>
@@ -18,6 +22,11 @@
 namespace gh {
 namespace app {
 
+// A block has inserted or taken keys: waits count their time limit from here.
+__device__ __forceinline__ void stamp(HeapState* st) {
+    if (threadIdx.x == 0) detail::st_relaxed(&st->progressNs, detail::globaltimer());
+}
+
 // Heap calls of the search loops, kept out of line.  Inlined into a search
 // loop, insertion and deleteMin (with their merges) compete for registers
 // with the loop's own state, and the compiler spills inside the merge
@@ -26,6 +35,7 @@ namespace app {
 template <typename H>
 __device__ __noinline__ void insert_keys(H heap, const unsigned long long* keys, int n, int heapOff) {
     heap.insertion(reinterpret_cast<const typename H::key_type*>(keys), n, heapOff, true);
+    stamp(heap.state);
 }
 
 // Inserts keys[0, n) (0 < n <= batchSize) and takes a batch, in one hold of
@@ -33,12 +43,15 @@ __device__ __noinline__ void insert_keys(H heap, const unsigned long long* keys,
 // block that comes out of a round with keys to insert goes into the next one
 // like this: it stays counted busy meanwhile, and the heap's serial part, which
 // bounds searches of several blocks, is passed once a round instead of twice.
+// While all keys fit one batch (a chain, a corridor) no other block sees any
+// and `busy` stands still.
 template <typename H>
 __device__ __noinline__ int exchange_batch(H heap, const unsigned long long* keys, int n, unsigned long long* out,
                                            typename H::key_type threshold, bool check, int heapOff) {
     int size = 0;
     heap.exchangeMin(reinterpret_cast<const typename H::key_type*>(keys), n, reinterpret_cast<typename H::key_type*>(out),
                      size, threshold, check, heapOff);
+    stamp(heap.state);
     return size;
 }
 
@@ -48,6 +61,7 @@ template <typename H>
 __device__ __noinline__ int take_batch(H heap, unsigned long long* out, typename H::key_type threshold, int heapOff) {
     int size = 0;
     heap.deleteMin(reinterpret_cast<typename H::key_type*>(out), size, threshold, heapOff);
+    if (size > 0) stamp(heap.state);
     return size;
 }
 
@@ -55,6 +69,7 @@ template <typename H>
 __device__ __noinline__ int take_batch(H heap, unsigned long long* out, int heapOff) {
     int size = 0;
     heap.deleteMin(reinterpret_cast<typename H::key_type*>(out), size, heapOff);
+    if (size > 0) stamp(heap.state);
     return size;
 }
 
@@ -77,8 +92,9 @@ struct NoThreshold {
 // smallest key is read without locks; while blocks are busy it is a hint
 // (a wrong one costs one empty deleteRoot or one early exit of this block,
 // while busy blocks carry on), and the last block to finish reads it with
-// no other block left inside the heap.  A wait with no change of busy for
-// longer than the heap's time limit records a timeout and stops.
+// no other block left inside the heap.  A wait with no change of busy and no
+// stamp of a working block for longer than the heap's time limit records a
+// timeout and stops.
 template <typename H, typename Threshold = NoThreshold>
 __device__ __forceinline__ bool wait_for_keys(const H& heap, int* word, const int* stop, int& lastBusy,
                                               unsigned long long& waitStart, Threshold threshold = {}) {
@@ -105,7 +121,7 @@ __device__ __forceinline__ bool wait_for_keys(const H& heap, int* word, const in
             if (detail::ld_relaxed(&st->err) != 0) { verdict = 1; break; }
             const unsigned long long now = detail::globaltimer();
             if (b != lastBusy || waitStart == 0) { lastBusy = b; waitStart = now; }
-            if (now - waitStart > static_cast<unsigned long long>(heap.timeoutNs)) {
+            if (heap.standsStill(waitStart, now)) {
                 heap.raise(kErrTimeout, kSiteLockPartial, 0, b);
                 verdict = 1;
                 break;

@@ -88,7 +88,8 @@ struct alignas(128) HeapState {
     int build;              // bulk insert: 1 when the reserved targets are filled by a heap build (k_build)
     int buildNext;          // heap build: next node to take, counting down
     int delStop;            // bulk deletes: set by the block that found nothing more to take
-    int pad2[6];
+    unsigned long long progressNs;  // applications: when a block last finished an operation (globaltimer; 0: none stamped)
+    int pad2[4];
     unsigned long long appStats[8];  // applications: counters (e.g. pops, expansions, relaxations)
 };
 
@@ -129,6 +130,11 @@ __device__ __forceinline__ int ld_relaxed(const int* p) {
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ int ld_acquire(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -136,6 +142,9 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 }
 __device__ __forceinline__ void st_relaxed(int* p, int v) {
     asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void st_release(int* p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -528,6 +537,13 @@ struct Heap {
         }
     }
 
+    // Whether the time limit has passed since t0 and since the last stamp of
+    // the application that runs on the heap.
+    __device__ __forceinline__ bool standsStill(unsigned long long t0, unsigned long long now) const {
+        return static_cast<long long>(now - t0) > timeoutNs &&
+               static_cast<long long>(now - detail::ld_relaxed(&state->progressNs)) > timeoutNs;
+    }
+
     // Periodic check inside a wait: false once the time limit has passed
     // (the error is raised) or another block has already raised one.
     __device__ __forceinline__ bool keep_waiting(unsigned long long& t0, unsigned it, int site, int nodeIdx,
@@ -535,7 +551,7 @@ struct Heap {
         if ((it & 15u) != 15u) return true;
         const unsigned long long now = detail::globaltimer();
         if (t0 == 0) t0 = now;
-        if (now - t0 > static_cast<unsigned long long>(timeoutNs)) {
+        if (standsStill(t0, now)) {
             raise(kErrTimeout, site, nodeIdx, seen);
             return false;
         }

@@ -24,7 +24,9 @@ modelled here at the level of those atomic steps:
   read before it is written or overwritten before it is read.
 * termination of a search (gpuheap_gb300/csrc/worklist.cuh): blocks that
   share one heap count themselves busy while they hold work; the search
-  must end exactly when the work is done, with no block left waiting.
+  must end exactly when the work is done, with no block left waiting; a
+  block may stay busy over many rounds, and the others' time limit must
+  not take that for a hang.
 * the retrieving heap's steal (include/gpuheap_retrieve.cuh; reference
   applications/sssp_longfei_new/heap.cuh:20-35, 147-199, 338-380): a
   retrieve that needs the last node while an insert is still on its way
@@ -428,6 +430,72 @@ def termination_model(blocks=2, depth=2, count_while_waiting=False):
             raise Violation(f"search ended with heap {g.heap}, busy {g.busy}, {g.processed}/{total} units", trace)
 
     return (TermState(heap=(depth,), busy=0, processed=0), tuple(["wait"] * blocks)), actors, final
+
+
+# --------------------------------------------------------------------------
+# a block that stays busy over rounds, and the time limit of the others
+
+RoundsState = namedtuple("RoundsState", "heap busy rounds timeouts")
+
+
+def busy_rounds_model(waiters=2, rounds=3, stamps=True, hangs=False):
+    """The time limit of `wait_for_keys` beside a block that keeps the whole
+    frontier to itself (gpuheap_gb300/csrc/worklist.cuh `exchange_batch`):
+    it takes one unit, passes its keys through the heap `rounds` times in
+    one hold each, stamping HeapState::progressNs after each (the model's
+    clock is the count of rounds), and uncounts itself at the end; the heap
+    looks empty and busy is 1 all along.
+
+    A waiting block opens a window when it sees busy change and may find it
+    expired at any time, provided a busy block that works has finished a
+    round or left since it was opened (a round takes less than the time
+    limit).  Expired: a stamp later than the window's start opens a new one
+    (`standsStill`), else a time-out.  Invariant: no time-out beside a block that
+    works.  With `hangs` the busy block stops for good after its first
+    round; then every waiting block must time out.  stamps=False plants the
+    mistake of looking at busy alone.  The same rule serves a block that
+    loses the race for node 0 to a working one."""
+
+    def worker(g, pc, trace):
+        if pc == "take":
+            return [("takes the unit, busy = 1", _set(g, heap=0, busy=1), ("exchange", rounds))]
+        _, left = pc
+        if hangs and left < rounds:
+            return []
+        if left == 0:
+            return [("busy -= 1", _set(g, busy=0), None)]
+        return [("exchanges, stamps", _set(g, rounds=g.rounds + 1), ("exchange", left - 1))]
+
+    def waiter(g, pc, trace):
+        if pc == "start":  # the search has begun: the unit is out of the heap
+            return [("opens a window", g, ("wait", g.busy, g.rounds))] if not g.heap else []
+        _, busy0, rounds0 = pc
+        moves = []
+        if g.busy == 0:
+            return [("heap empty, busy 0: leaves", g, None)]
+        if g.busy != busy0:
+            moves.append(("busy changed: new window", g, ("wait", g.busy, g.rounds)))
+        if g.rounds != rounds0 or (hangs and g.rounds):
+            if stamps and g.rounds != rounds0:
+                moves.append(("expired, stamped since: new window", g, ("wait", g.busy, g.rounds)))
+            elif hangs:
+                moves.append(("times out", _set(g, timeouts=g.timeouts + 1), None))
+            else:
+                raise Violation("time-out beside a block that works", list(trace) + ["waiter:times out"])
+        return moves
+
+    def named(i):
+        def act(g, pc, trace):
+            return waiter(g, pc, trace)
+        act.__name__ = f"waiter{i}"
+        return act
+
+    def final(g, trace):
+        if g.heap or g.busy or g.timeouts:
+            raise Violation(f"ended with heap {g.heap}, busy {g.busy}, {g.timeouts} time-outs", trace)
+
+    g0 = RoundsState(heap=1, busy=0, rounds=0, timeouts=0)
+    return (g0, ("take",) + ("start",) * waiters), [worker] + [named(i) for i in range(waiters)], final
 
 
 # --------------------------------------------------------------------------
