@@ -264,6 +264,12 @@ __device__ __forceinline__ K lds(unsigned addr) {
 // addresses sa and sb (n keys each, d + IPT <= 2n): a binary search on the
 // diagonal d finds the split (a wins ties, as heap/heaputil.cuh:99-158
 // does), IPT sequential steps fill the registers.
+// 8-byte keys: one load a step from the run that was taken from.  With a load
+// in either branch, nvcc 13.0 compiled some callers so that a key left with
+// the low word of its successor (exchangeMin in a user's kernel, bottom-up,
+// any batch size; not at -Xptxas -O0 and not with plain loads).  Sort of 2^24
+// u64 keys 1.96 -> 1.84 ms.  4-byte keys, whole registers each, keep the
+// branches: sort of 2^28 u32 keys 12.39 ms, 12.55 with the one load.
 template <typename K, int IPT>
 __device__ __forceinline__ void merge_run(unsigned sa, unsigned sb, int n, int d, K (&r)[IPT]) {
     constexpr unsigned S = sizeof(K);
@@ -281,8 +287,17 @@ __device__ __forceinline__ void merge_run(unsigned sa, unsigned sb, int n, int d
     for (int k = 0; k < IPT; ++k) {
         const bool ta = (j >= n) || (i < n && av <= bv);
         r[k] = ta ? av : bv;
-        if (ta) { ++i; av = lds<K>(sa + S * (i < n ? i : n - 1)); }
-        else { ++j; bv = lds<K>(sb + S * (j < n ? j : n - 1)); }
+        if constexpr (sizeof(K) == 8) {
+            i += ta;
+            j += !ta;
+            const int at = ta ? i : j;
+            const K nx = lds<K>((ta ? sa : sb) + S * (at < n ? at : n - 1));
+            av = ta ? nx : av;
+            bv = ta ? bv : nx;
+        } else {
+            if (ta) { ++i; av = lds<K>(sa + S * (i < n ? i : n - 1)); }
+            else { ++j; bv = lds<K>(sb + S * (j < n ? j : n - 1)); }
+        }
     }
 }
 
