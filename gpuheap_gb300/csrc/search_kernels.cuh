@@ -572,6 +572,11 @@ __device__ bool run_sssp(const H& heap, Inst* in, unsigned char* smem, int heapO
             break;
         }
         int size = 0;
+        if (kept && gh::app::crowded(heap, &ctl[2], kept)) {
+            flush_rest(heap, emit, &ctl[1], heapOff, inserted);
+            gh::app::batch_done(heap.state);
+            kept = 0;
+        }
         if (kept) {
             size = exchange_rest(heap, emit, &ctl[1], kept, batch, ~0ull, heapOff, inserted, false);
         } else {

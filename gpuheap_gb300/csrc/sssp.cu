@@ -106,6 +106,14 @@ __global__ void __launch_bounds__(1024) k_sssp(H heap, const long long* __restri
     int kept = 0;  // keys of the last round still to be inserted (the block stays busy)
     for (;;) {
         int size;
+        if (kept && gh::app::crowded(heap, &ctl[2], kept)) {
+            gh::app::insert_keys(heap, emit, kept, heapOff);
+            inserted += kept;
+            kept = 0;
+            __syncthreads();
+            if (tid == 0) ctl[1] = 0;
+            gh::app::batch_done(st);
+        }
         if (kept) {
             size = gh::app::exchange_batch(heap, emit, kept, batch, heap.init_limits, false, heapOff);
             inserted += kept;

@@ -38,8 +38,8 @@ def strip(length, width, seed):
 
 
 @pytest.mark.parametrize("variant", ["bottomup", "topdown"])
-@pytest.mark.parametrize("length,width,B", [(20000, 1, 256), (6000, 100, 2048)])
-def test_sssp_on_a_chain_and_a_strip(variant, length, width, B):
+@pytest.mark.parametrize("length,width,B", [(20000, 1, 256), (6000, 100, 2048), (400, 400, 256)])
+def test_sssp_on_chains_strips_and_grids(variant, length, width, B):
     rowptr, col, w = strip(length, width, length)
     g = gsssp.Graph(rowptr.size - 1, torch.from_numpy(rowptr).cuda(), torch.from_numpy(col).cuda(),
                     torch.from_numpy(w.view(np.int32)).cuda())
