@@ -458,6 +458,15 @@ __device__ __forceinline__ void sort_batch(const K* src, int size, K* s, int n, 
     }
 }
 
+// The same by the bitonic network, for any block.
+template <typename K>
+__device__ __forceinline__ void sort_network(const K* src, int size, K* s, int n, K pad) {
+    for (int i = static_cast<int>(threadIdx.x); i < n; i += static_cast<int>(blockDim.x)) s[i] = i < size ? src[i] : pad;
+    __syncthreads();
+    bitonic_sort(s, n);
+    __syncthreads();
+}
+
 // R chosen at run time: the keys a thread has when the block's threads share
 // the batch (1 to 8); more keys a thread, and blocks of less than a warp
 // (the retrieving heap's at batch 16), take the bitonic network.
@@ -468,12 +477,7 @@ __device__ __forceinline__ void sort_batch_rt(const K* src, int size, K* s, int 
     else if (per == 2) sort_batch<K, 2>(src, size, s, n, pad);
     else if (per == 4) sort_batch<K, 4>(src, size, s, n, pad);
     else if (per == 8) sort_batch<K, 8>(src, size, s, n, pad);
-    else {
-        for (int i = static_cast<int>(threadIdx.x); i < n; i += static_cast<int>(blockDim.x)) s[i] = i < size ? src[i] : pad;
-        __syncthreads();
-        bitonic_sort(s, n);
-        __syncthreads();
-    }
+    else sort_network<K>(src, size, s, n, pad);
 }
 
 template <typename K>
@@ -538,6 +542,10 @@ struct Heap {
 
     // items[0, size) sorted into s0, padded with init_limits to a batch.
     __device__ __forceinline__ void sortBatch(const K* items, int size, K* s0) const {
+        // a search of batch size 32 may run on blocks of 16 threads, which have no warp to sort in registers
+        if constexpr (IPT == 4 && sizeof(K) == 8) {
+            if (blockDim.x < 32) { detail::sort_network<K>(items, size, s0, batchSize, init_limits); return; }
+        }
         if constexpr (IPT > 0) detail::sort_batch<K, (IPT > 2 ? IPT / 2 : 1)>(items, size, s0, batchSize, init_limits);
         else detail::sort_batch_rt<K>(items, size, s0, batchSize, init_limits);
     }
