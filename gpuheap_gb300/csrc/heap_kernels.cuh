@@ -8,6 +8,7 @@
 #include <atomic>
 
 #include "gpuheap_device.cuh"
+#include "insert_plan.h"
 
 namespace gh {
 namespace impl {
@@ -71,33 +72,28 @@ __global__ void __launch_bounds__(1024) k_insert(H h, const K* __restrict__ keys
     }
 }
 
-// A bulk insert that makes the heap at most this many times the new batches
-// is a heap build (k_build); one that adds fewer batches inserts them one by
-// one (k_insert_reserved).  Measured on GB300, microseconds for m batches
-// into a heap of N (build / one by one): u32, batch 2048, N = 16384: m = 64
-// 264 / 160, m = 256 174 / 462; batch 1024, N = 1024: m = 16 111 / 96,
-// m = 64 87 / 236; batch 256, N = 8192: m = 64 155 / 85, m = 256 109 / 181;
-// u64, batch 1024, N = 4096: m = 16 266 / 123, m = 64 143 / 304.  The lines
-// cross at N / m = 50 to 160.
-constexpr int kBuildRatio = 48;
-
 // Bulk insert of `m` full batches, step 1 (one thread): with the partial
 // buffer empty, no error recorded and room for all of them, reserve targets
 // batchCount+1 .. batchCount+m (batchCount moves past them now, as m
-// node-0 hand-offs would have moved it) and choose how to fill them;
+// node-0 hand-offs would have moved it) and choose how to fill them
+// (build_pays);
 // otherwise reserve nothing and the insert kernel takes node 0 per batch as
 // the reference does.
-__device__ __forceinline__ void reserve_targets(HeapState* st, int batchNum, long long m) {
+template <typename H>
+__device__ __forceinline__ void reserve_targets(HeapState* st, int batchNum, int nodeBytes, long long m) {
     const int bc = st->batchCount;
     const bool ok = m > 0 && st->err == 0 && st->partialBufferSize == 0 && bc + m <= batchNum;
     st->resvBase = bc;
     st->resvCount = ok ? static_cast<int>(m) : 0;
     st->resvTurn = bc + 1;
-    st->build = ok && bc + m <= kBuildRatio * m;
+    st->build = ok && build_pays(H::kVariant == kTopDown, nodeBytes, m, bc);
     st->buildNext = bc + static_cast<int>(ok ? m : 0);
     if (ok) st->batchCount = bc + static_cast<int>(m);
 }
-static __global__ void k_reserve(HeapState* st, int batchNum, long long m) { reserve_targets(st, batchNum, m); }
+template <typename H>
+__global__ void k_reserve(HeapState* st, int batchNum, int nodeBytes, long long m) {
+    reserve_targets<H>(st, batchNum, nodeBytes, m);
+}
 
 // Step 2: the reserved targets' lock words take the state an insert holds
 // its target in (top-down TARGET, bottom-up INUSE), so that an insert that
@@ -118,12 +114,13 @@ __device__ __forceinline__ void mark_targets(const HeapState* st, int* status) {
 }
 template <typename H>
 __global__ void k_mark_reserved(const HeapState* st, int* status) { mark_targets<H>(st, status); }
-// Both steps by one block, for heaps of up to kReserveOne nodes (a launch
-// less, 2 us; one block marks 16 nodes a thread in about that).
+// Both steps by one block where at most kReserveOne nodes can be marked (a
+// launch less, 2 us; one block marks 16 nodes a thread in about that).
 constexpr int kReserveOne = 16384;
 template <typename H>
-__global__ void __launch_bounds__(1024) k_reserve_mark(HeapState* st, int* status, int batchNum, long long m) {
-    if (threadIdx.x == 0) reserve_targets(st, batchNum, m);
+__global__ void __launch_bounds__(1024) k_reserve_mark(HeapState* st, int* status, int batchNum, int nodeBytes,
+                                                       long long m) {
+    if (threadIdx.x == 0) reserve_targets<H>(st, batchNum, nodeBytes, m);
     __syncthreads();
     mark_targets<H>(st, status);
 }

@@ -169,17 +169,19 @@ cudaError_t launch_insert(const LaunchArgs& a, const K* keys, long long n, int c
         const long long m = (a.reserve && chunk == B) ? n / B : 0;
         if (m > 0) {
             if (!a.prepared) {
-                if (a.d->batchNum <= kReserveOne) {
-                    k_reserve_mark<H><<<1, 1024, 0, a.stream>>>(a.d->state, a.d->status, a.d->batchNum, m);
+                const int nodeBytes = B * static_cast<int>(sizeof(K));
+                if (a.d->batchNum <= kReserveOne || kBuildRatio * m <= kReserveOne) {
+                    k_reserve_mark<H><<<1, 1024, 0, a.stream>>>(a.d->state, a.d->status, a.d->batchNum, nodeBytes, m);
                 } else {
-                    k_reserve<<<1, 1, 0, a.stream>>>(a.d->state, a.d->batchNum, m);
+                    k_reserve<H><<<1, 1, 0, a.stream>>>(a.d->state, a.d->batchNum, nodeBytes, m);
                     count_launch();
                     const long long mb = (m + 255) / 256;
                     k_mark_reserved<H><<<static_cast<int>(mb < 1024 ? mb : 1024), 256, 0, a.stream>>>(a.d->state, a.d->status);
                 }
                 count_launch();
             }
-            cudaError_t e = launch_build<K>(a, keys, m, H::kHasPartialBuffer ? static_cast<int>(n - m * B) : 0);
+            cudaError_t e = cudaSuccess;
+            if (a.prepared || m >= kBuildLeast) e = launch_build<K>(a, keys, m, H::kHasPartialBuffer ? static_cast<int>(n - m * B) : 0);
             if (e != cudaSuccess) return e;
             if (a.prepared && (H::kHasPartialBuffer || n == m * B)) return cudaSuccess;
             if (!a.prepared) {

@@ -74,8 +74,8 @@ gh_status gh_heap_set_owner_depth(gh_heap* h, int depth);
  * chunk <= batch_size), spread over the heap's grid.  With chunk = batch_size
  * and the partial buffer empty, the full batches' target nodes are reserved
  * in one step before they are inserted, so they do not take node 0 one at a
- * time; when they are at least 1/48 of the nodes the heap then has, they and
- * their ancestors are sifted from the bottom up (a heap build) instead of
+ * time; when they are many and a good part of the nodes the heap then has
+ * (1/6 to 1/48, by the node's size), they and their ancestors are sifted from the bottom up (a heap build) instead of
  * one insertion after another.  The result is a heap of the same keys and
  * node count.  No other operation may use the heap during the call (the reference's
  * tests run insertKernel as a phase of its own). */
