@@ -33,11 +33,11 @@ constexpr int kBuildRatio = 48;
 //     n = 248 60 / 56; m = 16, n = 736 68 / 86
 // The lines cross near n = m^3 / 16 while there are few batches (m^3 / 32 for
 // nodes below 512 bytes); small nodes, whose inserts cost little, stop at 6 to
-// 24 times the batches (more once the inserts contend, from 128 on).  Top-down inserts go one at a time through
-// the root and lose sooner.
+// 24 times the batches (more once the inserts contend, from 128 on).  Top-down
+// inserts go one at a time through the root and lose sooner, near m^3 / 4.
 GH_PLAN_HD inline bool build_pays(bool topDown, long long nodeBytes, long long m, long long n) {
     if (m < kBuildLeast || n + m > kBuildRatio * m) return false;
-    if (m < 64 && (topDown ? 8 : nodeBytes < 512 ? 32 : 16) * n > m * m * m) return false;
+    if (m < 64 && (topDown ? 4 : nodeBytes < 512 ? 32 : 16) * n > m * m * m) return false;
     if (topDown) return true;
     const long long most = nodeBytes < 128 ? 6 : nodeBytes < 512 ? 12 : nodeBytes < 1024 ? 24 : kBuildRatio;
     return n + m <= most * m * (m < 128 ? 128 : m < 1024 ? m : 1024) / 128;

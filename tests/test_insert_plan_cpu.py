@@ -44,7 +44,7 @@ def test_a_few_batches_into_a_small_heap_go_one_by_one(pays):
 
 @pytest.mark.parametrize("top,node,m,most", [(0, 2048, 4, 4), (0, 2048, 8, 32), (0, 2048, 16, 256), (0, 8192, 63, 47 * 63),
                                              (0, 64, 8, 16), (0, 64, 64, 5 * 64), (0, 64, 512, 23 * 512), (0, 512, 64, 23 * 64),
-                                             (0, 8192, 1 << 20, 47 << 20), (1, 64, 4, 8), (1, 64, 16, 512), (1, 64, 64, 47 * 64)])
+                                             (0, 8192, 1 << 20, 47 << 20), (1, 64, 4, 16), (1, 64, 16, 47 * 16), (1, 64, 64, 47 * 64)])
 def test_edges(pays, top, node, m, most):
     assert pays([(top, node, m, most), (top, node, m, most + 1), (top, node, m, 0)]) == [1, 0, 1]
 
