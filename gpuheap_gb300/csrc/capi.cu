@@ -265,6 +265,7 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
     if (chunk == 0) chunk = h->d.batchSize;
     if (chunk < 1 || chunk > h->d.batchSize) return GH_ERR_INVALID;
     if (n == 0) return GH_OK;
+    h->d.restored = 0;
     const gh::impl::LaunchArgs a = args_of(h, static_cast<cudaStream_t>(stream));
     return with_key(h, [&](auto k) {
         using K = decltype(k);
@@ -400,6 +401,7 @@ gh_status delete_bulk(gh_heap* h, void* out_dev, long long max_keys, const void*
     if (n_out) h->words->dc = -1;  // a sort that does not start leaves it
     else a.words = nullptr;
     gh_status st = launch();
+    h->d.restored = 0;
     if (!kept) cudaFreeAsync(a.tmp, s);
     if (st != GH_OK || !n_out) return st;
     GH_CUDA(cudaStreamSynchronize(s));
@@ -432,6 +434,7 @@ gh_status gh_heap_delete_below(gh_heap* h, void* out_dev, long long max_keys, co
 gh_status gh_heap_gc(gh_heap* h, const void* threshold, long long* kept, void* stream) {
     gh::trace::Range range_("gh_heap_gc");
     if (!h) return GH_ERR_INVALID;
+    h->d.restored = 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // the used nodes, after the stream's work (the reference's invalidFilter
     // reads batchCount the same way, artifacts/astar/gc.cuh:153-154)
@@ -495,6 +498,7 @@ gh_status gh_heap_concurrent(gh_heap* h, const void* keys_dev, long long n, int 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     gh::impl::LaunchArgs a = args_of(h, s);
     if (a.grid < 2) a.grid = 2;  // one inserting and one deleting block at least
+    h->d.restored = 0;
     const long long deletes = n / h->d.batchSize;
     const int lim = static_cast<int>(std::min<long long>(max_keys, INT_MAX));
     gh::impl::k_set_output<<<1, 32, 0, s>>>(h->d.state, 0, lim);

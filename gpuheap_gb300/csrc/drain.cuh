@@ -85,9 +85,11 @@ inline size_t drain_bytes(int blocks) { return sizeof(DrainCtl) + sizeof(unsigne
 // Fewest full nodes a drain takes on.  A single tile takes about as long as
 // four plain deletes and their launch; 1024 nodes of 1024 keys take 82 us,
 // and the owner mode 4.4 us for each delete, so the owner mode is never the
-// faster way to empty a heap.  Up to 256 nodes it stays for a restored heap,
-// whose deletes are replayed one by one: its counters (gh_heap_owner_stats)
-// are read to see which sift steps that very heap takes.
+// faster way to empty a heap.  Up to 256 nodes it stays for the first bulk
+// operation on a restored heap, whose deletes are replayed one by one: its
+// counters (gh_heap_owner_stats) are read to see which sift steps that very
+// heap takes.  A program that restores a snapshot and goes on pays for that
+// once (200 nodes of 1024 keys 0.86 ms, 0.07 as a sort).
 constexpr int kDrainNodes = 4;
 constexpr int kDrainNodesRestored = 256;
 inline int drain_nodes(const Desc& d) { return d.mbox && d.restored ? kDrainNodesRestored : kDrainNodes; }

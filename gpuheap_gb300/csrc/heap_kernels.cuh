@@ -33,7 +33,7 @@ struct Desc {
     int ownerDepth;  // owner-mode resident depth: -1 automatic, 0 off, else 2..4
     void* drain;  // whole-heap deletes: DrainCtl and the digit counts (null: none)
     int drainBlocks;  // blocks the counts have room for
-    int restored;  // the heap's content was put back by gh_heap_restore and not reset since
+    int restored;  // gh_heap_restore has put the heap's content back and no bulk operation or reset has followed
 };
 
 // What a call that waits for its result reads: in pinned host memory, written

@@ -86,8 +86,8 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
  * are written in ascending order (HEAP_SORT) to out_dev[0, *n_out).  When
  * n_out is not NULL the call synchronizes the stream to read the count.  A
  * heap that max_keys holds whole is emptied by one radix sort between its
- * nodes and out_dev (from 4 nodes on; a heap that gh_heap_restore filled from
- * 256 on where the batch size has an owner mode) unless an owner depth was
+ * nodes and out_dev (from 4 nodes on; the first bulk operation after
+ * gh_heap_restore from 256 on where the batch size has an owner mode) unless an owner depth was
  * chosen; the nodes then all hold
  * init_limits.  With n_out, a call that takes many batches and leaves others
  * sorts too, between the nodes and a scratch array of the heap's keys (up to
