@@ -53,6 +53,14 @@ modelled here at the level of those atomic steps:
   lock is released while a retrieve reads the heap.
 * the FIFO's whole-call push (fifo.cu `k_fifo_bulk_push`): the last block
   to count itself in publishes what the grid copied.
+* a bulk delete's end (`bulkStop`): the block that finds nothing more says
+  so, and the others give their tickets up.
+* the exchange's last node (`exchangeTry`), taken before it is known to be
+  needed and given back as it was found.
+* the locks of the next level (`sift_loop`, `insert_bottomup`), taken or
+  tried before the last level is released.
+* the heap build (heap_kernels.cuh `k_build`): nodes in descending order,
+  sifts down hand over hand.
 
 A spin wait is a step that is enabled only when its condition holds, so a
 state where no actor can move but some have not finished is a deadlock.
@@ -1551,3 +1559,252 @@ def fifo_bulk_model(blocks=3, last_commits=True, arrive_after_copy=True):
     g0 = BulkState(slots=(False,) * blocks, arrived=0, write=0, got=0)
     start = "copy" if arrive_after_copy else "arrive_first"
     return (g0, tuple(start for _ in range(blocks)) + (0,)), [block(b) for b in range(blocks)] + [popper], final
+
+
+# --------------------------------------------------------------------------
+# the exchange's last node, taken and given back unchanged
+
+GiveState = namedtuple("GiveState", "x p ver seen_i")
+
+
+def exchange_giveback_model(back_as_found=True, unchanged=True, refuse=True):
+    """Bottom-up `exchangeTry` (include/gpuheap_device.cuh) beside a parked
+    insert: the exchange takes the last node x with atomicMax before it knows
+    whether it will need it, and when the threshold refuses it releases x
+    with the state it found, the node untouched.
+
+    * `ins` has parked x with its ticket and waits for p (held by `holder`),
+      then takes x back and trusts its cached batch if it finds its ticket.
+    * `exch` takes x; refused, it gives x back, else it uses x up: writes it
+      and releases it AVAIL.
+
+    An insert that trusts asserts that nobody wrote x since its park.
+    Planted: the node is written before it is given back as found
+    (unchanged=False).  back_as_found=False (always AVAIL) is safe: the
+    insert then reloads x, which costs a load."""
+    tag = PARK_BASE
+
+    def ins(g, pc, trace):
+        if pc == "lock_p":
+            return [("lock p", _set(g, p=INUSE), "retake")] if g.p == AVAIL else []
+        if pc == "retake":
+            if g.x == INUSE:
+                return []
+            if g.x == tag and g.ver != g.seen_i:
+                raise Violation("insert trusted a stale copy of its parked node", list(trace) + ["ins:retake"])
+            return [(f"retake x (found {g.x})", _set(g, x=INUSE), "write")]
+        if pc == "write":
+            return [("write, release x and p", _set(g, x=AVAIL, p=AVAIL, ver=g.ver + 1), None)]
+        return []
+
+    def holder(g, pc, trace):
+        return [("release p", _set(g, p=AVAIL), None)]
+
+    def exch(g, pc, trace):
+        if pc == "take":
+            return [(f"take x (found {g.x})", _set(g, x=INUSE), ("held", g.x))] if g.x != INUSE else []
+        _, found = pc
+        if refuse:
+            ver = g.ver if unchanged else g.ver + 1
+            return [("refused: give x back", _set(g, x=found if back_as_found else AVAIL, ver=ver), None)]
+        return [("use x up, release AVAIL", _set(g, x=AVAIL, ver=g.ver + 1), None)]
+
+    def final(g, trace):
+        if g.x != AVAIL or g.p != AVAIL:
+            raise Violation(f"a lock word left taken (x={g.x}, p={g.p})", trace)
+
+    g0 = GiveState(x=tag, p=INUSE, ver=0, seen_i=0)
+    return (g0, ("lock_p", "hold", "take")), [ins, holder, exch], final
+
+
+# --------------------------------------------------------------------------
+# a bulk delete's end: the block that finds nothing more says so
+
+StopState = namedtuple("StopState", "items ticket serving holder stop taken")
+
+
+def delete_stop_model(blocks=3, items=2, lookers=None):
+    """`takeTurn` and `bulkStop` (include/gpuheap_device.cuh): a block leaves
+    when it reads delStop before it draws a ticket or while it waits for it;
+    the block that holds node 0 and finds nothing to take sets delStop.
+    A block that leaves while it waits gives its ticket up, and no later one
+    is served, so every waiting block must look at delStop (lookers=1 plants
+    the mistake that only the first block does).
+
+    Invariants: every item is taken, node 0 has one holder at a time and
+    every block leaves."""
+
+    def block(i):
+        def act(g, pc, trace):
+            step, t = pc
+            if step == "start":
+                if g.stop:
+                    return [("reads delStop: leaves", g, None)]
+                return [("reads no delStop", g, ("draw", None))]
+            if step == "draw":
+                return [(f"draws ticket {g.ticket}", _set(g, ticket=g.ticket + 1), ("wait", g.ticket))]
+            if step == "wait":
+                moves = []
+                if g.serving == t:
+                    moves.append(("served", g, ("lock", t)))
+                elif g.stop and (lookers is None or i < lookers):
+                    moves.append(("reads delStop: leaves", g, None))
+                return moves
+            if step == "lock":
+                return [("locks node 0", _set(g, holder=i), ("pass", t))] if g.holder == -1 else []
+            if step == "pass":
+                return [("passes the turn", _set(g, serving=t + 1), ("take", t))]
+            if g.items == 0:
+                return [("nothing left: delStop, unlocks", _set(g, stop=True, holder=-1), None)]
+            return [("takes a batch, unlocks", _set(g, items=g.items - 1, taken=g.taken + 1, holder=-1), ("start", None))]
+        act.__name__ = f"b{i}"
+        return act
+
+    def final(g, trace):
+        if g.items or g.taken != items or g.holder != -1:
+            raise Violation(f"{g.taken} of {items} batches taken, holder {g.holder}", trace)
+
+    g0 = StopState(items=items, ticket=0, serving=0, holder=-1, stop=False, taken=0)
+    return (g0, tuple(("start", None) for _ in range(blocks))), [block(i) for i in range(blocks)], final
+
+
+# --------------------------------------------------------------------------
+# locks of the next level taken before the last level is released
+
+NextState = namedtuple("NextState", "lock")
+
+
+def next_level_model(levels=4, sifts=2, inserts=1, try_once=True):
+    """One path of a bottom-up heap, nodes 0 (the root) .. levels - 1.
+
+    A sift (`sift_loop`) holds node k; at each level one warp takes the child
+    k + 1 (waiting for it, parked or not) while thread 0 releases node k - 1:
+    the two happen in either order, both before the next level.  A bubbling
+    insert (`insert_bottomup`) holds node k, tries its parent once while
+    thread 0 releases node k + 1, and parks k before it waits for the parent.
+    try_once=False plants the mistake of waiting for the parent there.
+
+    Invariant: everything ends with every word free, whatever the order."""
+
+    def sift(i):
+        def act(g, pc, trace):
+            w = g.lock
+            step, k, taken, released = pc
+            if step == "start":
+                return [("takes the root", _set(g, lock=_put(w, 0, INUSE)), ("level", 0, False, True))] if w[0] == AVAIL else []
+            moves = []
+            if not released:
+                moves.append((f"releases {k - 1}", _set(g, lock=_put(w, k - 1, AVAIL)), (step, k, taken, True)))
+            if k + 1 == levels:
+                if released:
+                    return [(f"releases {k}", _set(g, lock=_put(w, k, AVAIL)), None)]
+                return moves
+            if not taken and w[k + 1] != INUSE:
+                moves.append((f"takes {k + 1} (found {w[k + 1]})", _set(g, lock=_put(w, k + 1, INUSE)), (step, k, True, released)))
+            if taken and released:
+                moves.append(("next level", g, (step, k + 1, False, False)))
+            return moves
+        act.__name__ = f"sift{i}"
+        return act
+
+    def insert(i):
+        tag = PARK_BASE + i
+
+        def act(g, pc, trace):
+            w = g.lock
+            step, k, tried, released = pc
+            if step == "start":
+                last = levels - 1
+                return [("claims the last node", _set(g, lock=_put(w, last, INUSE)), ("level", last, None, True))] if w[last] == AVAIL else []
+            if step == "level":
+                if k == 0:
+                    if released:
+                        return [("releases the root", _set(g, lock=_put(w, 0, AVAIL)), None)]
+                    return [("releases 1", _set(g, lock=_put(w, 1, AVAIL)), (step, k, tried, True))]
+                moves = []
+                if not released:
+                    moves.append((f"releases {k + 1}", _set(g, lock=_put(w, k + 1, AVAIL)), (step, k, tried, True)))
+                if tried is None:
+                    if w[k - 1] == AVAIL:
+                        moves.append((f"takes {k - 1}", _set(g, lock=_put(w, k - 1, INUSE)), (step, k, True, released)))
+                    elif try_once:
+                        moves.append((f"{k - 1} is held", g, (step, k, False, released)))
+                if tried is not None and released:
+                    if tried:
+                        moves.append(("merges, up a level", g, (step, k - 1, None, False)))
+                    else:
+                        moves.append((f"parks {k}", _set(g, lock=_put(w, k, tag)), ("parked", k, None, True)))
+                return moves
+            if step == "parked":
+                return [(f"takes {k - 1}", _set(g, lock=_put(w, k - 1, INUSE)), ("retake", k, None, True))] if w[k - 1] == AVAIL else []
+            return [(f"takes {k} back", _set(g, lock=_put(w, k, INUSE)), ("level", k, True, True))] if w[k] != INUSE else []
+        act.__name__ = f"insert{i}"
+        return act
+
+    def final(g, trace):
+        if any(v != AVAIL for v in g.lock):
+            raise Violation(f"lock words left {g.lock}", trace)
+
+    g0 = NextState(lock=(AVAIL,) * levels)
+    start = ("start", 0, None, True)
+    return (g0, (start,) * (sifts + inserts)), [sift(i) for i in range(sifts)] + [insert(i) for i in range(inserts)], final
+
+
+# --------------------------------------------------------------------------
+# the heap build: nodes in descending order, sifts hand over hand
+
+BuildState = namedtuple("BuildState", "next lock heap")
+
+
+def build_model(nodes=6, blocks=2, descending=True):
+    """k_build (gpuheap_gb300/csrc/heap_kernels.cuh) on a heap of `nodes` new
+    batches, every word held from the start.  A block takes the next node
+    from a counter; a leaf is written and released, an inner node sifted: the
+    block waits for both children's words (a child's own sift releases it
+    after its first level), releases the node and goes down into either.
+
+    Invariants: a sift only takes nodes whose own build has begun to release
+    them, every node is released once the build ends and no block waits
+    forever, with fewer blocks than nodes too.  descending=False plants the
+    wrong order: the blocks wait for children that nobody takes."""
+    order = list(range(nodes, 0, -1)) if descending else list(range(1, nodes + 1))
+
+    def block(i):
+        def act(g, pc, trace):
+            step, v = pc
+            if step == "next":
+                if g.next == len(order):
+                    return [("no node left", g, None)]
+                return [(f"takes node {order[g.next]}", _set(g, next=g.next + 1), ("sift", order[g.next]))]
+            kids = [c for c in (2 * v, 2 * v + 1) if c <= nodes]
+            if step == "sift":
+                free = [c for c in kids if g.lock[c] == AVAIL]
+                if len(free) < len(kids):
+                    # take what is free, as the lock warps do, and wait for the rest
+                    return [(f"takes {free[0]}", _set(g, lock=_put(g.lock, free[0], 100 + i)), ("sift", v))] if free else \
+                        ([("goes on", g, ("held", v))] if all(g.lock[c] == 100 + i for c in kids) else [])
+                if not kids:
+                    return [(f"releases leaf {v}", _set(g, lock=_put(g.lock, v, AVAIL), heap=_put(g.heap, v, True)), ("next", None))]
+                return [(f"takes {free[0]}", _set(g, lock=_put(g.lock, free[0], 100 + i)), ("sift", v))]
+            for c in kids:
+                if not g.heap[c]:
+                    raise Violation(f"node {v} met node {c} before its build", list(trace))
+            moves = []
+            freed = _put(g.lock, v, AVAIL)
+            heap = _put(g.heap, v, True)
+            for down in kids:  # the other child is released with the node
+                lock = freed
+                for c in kids:
+                    if c != down:
+                        lock = _put(lock, c, AVAIL)
+                moves.append((f"releases {v}, down to {down}", _set(g, lock=lock, heap=heap), ("sift", down)))
+            return moves
+        act.__name__ = f"b{i}"
+        return act
+
+    def final(g, trace):
+        if any(v != AVAIL for v in g.lock[1:]) or not all(g.heap[1:]):
+            raise Violation(f"lock words left {g.lock}", trace)
+
+    g0 = BuildState(next=0, lock=(AVAIL,) + (INUSE,) * nodes, heap=(True,) + (False,) * nodes)
+    return (g0, (("next", None),) * blocks), [block(i) for i in range(blocks)], final
