@@ -19,7 +19,8 @@
 //   * digits that all keys share (found with the first count) take no pass;
 //   * at the end the keys are in the output and the nodes hold init_limits
 //     again.  Every lock word is held meanwhile; one that is not free when
-//     the kernel starts leaves the work to the delete loops.
+//     the kernel starts leaves the work to the delete loops (no other
+//     operation may use the heap during a bulk delete).
 //
 // A bulk delete that takes many batches and leaves the rest sorts the same
 // way between the node array and a scratch array: the smallest keys go to
@@ -29,8 +30,9 @@
 //
 // Measured on GB300: 2^28 u32 keys 6.7 ms (611 ms in owner mode), 2^27 u64
 // 8.3 ms, 2^20 u32 82 us (3.8 ms), one tile about 20 us.  Bound by issue
-// slots: 2^26 u32 take 1.9 IPC at 28 % of DRAM bandwidth, most of it the
-// ranking's eight ballots a key; below 2^20 keys by the two grid barriers a
+// slots: 2^26 u32 take 1.96 IPC at 30 % of DRAM bandwidth, most of it the
+// ranking's eight ballots a key (64 registers a thread, 112 bytes spilled, 80
+// for 8-byte keys); below 2^20 keys by the two grid barriers a
 // pass (a third one, with the counts' scan spread over the grid, took 105 us
 // at 2^20 and gained nothing at any size).
 #pragma once
@@ -464,10 +466,11 @@ __global__ void __launch_bounds__(kDrainThreads, kDrainBlocksPerSM) k_drain(H h,
     // (sort_alone)
     const bool one = G == static_cast<int>(tiles), alone = tiles == 1;
 
-    // Take every lock word.  An operation still in flight holds one at any
-    // time (it locks the next node before it frees the last), so it makes
-    // this fail or waits until the end.  A thread stops at its first failure:
-    // the first `mine` of its words are its own.
+    // Take every lock word.  This finds words that are left taken; it does not
+    // make the sort safe beside another operation, which no bulk delete allows:
+    // counters and keys are read without waiting for all the words, so that an
+    // operation that ends meanwhile could leave its keys unseen.  A thread
+    // stops at its first failure: the first `mine` of its words are its own.
     const int stride = G * kDrainThreads;
     int mine = 0;
     for (int i = blk * kDrainThreads + tid; i <= bc; i += stride, ++mine)

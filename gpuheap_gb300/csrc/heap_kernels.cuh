@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(1024) k_reserve_mark(HeapState* st, int* statu
 // a step per level for each and every path meets at the top.  2^28 u32 keys,
 // batch 2048: 5.7 ms (112 ms one by one; 16.3 ms with the batches sorted by
 // a shared-memory bitonic network); 2^20, batch 1024: 91 us.  Bound by the
-// blocks' sort and merge instructions (2.45 IPC): 6.3 GB cross DRAM, 0.9 ms of
+// blocks' sort and merge instructions (2.48 IPC): 6.3 GB cross DRAM, 0.9 ms of
 // it.  8 keys a thread in the batch sort instead of 4 took 6.1 ms.  Node "0" is the ragged last batch (fewer than
 // batchSize keys), which only meets the root and the partial buffer.
 template <typename H, typename K>

@@ -53,8 +53,10 @@ gh_status gh_heap_reset(gh_heap* h, void* stream);
  * It turns a hang into GH_ERR_TIMEOUT.  The bulk drivers keep every wait
  * short: a bulk insert reserves its targets (no race for node 0), the blocks
  * of a bulk delete queue for node 0 by ticket, and an owner-mode delete's
- * waits last a few deletes.  Single operations and application kernels that
- * race many blocks on one heap's node 0 may need a longer limit. */
+ * waits last a few deletes.  In a search (gh_sssp, batched, served) a wait
+ * counts from the last insert or take of any of its blocks.  Single operations
+ * and application kernels of your own that race many blocks on one heap's
+ * node 0 may need a longer limit. */
 gh_status gh_heap_set_timeout(gh_heap* h, double seconds);
 /* Threads per block for the bulk entry points (0 = automatic: 16-byte merge
  * runs per thread); a power of two in [32, 1024] with 2*batch_size/threads
@@ -83,8 +85,8 @@ gh_status gh_heap_insert(gh_heap* h, const void* keys_dev, long long n, int chun
 
 /* deleteKernel (test/heap_test.cu:60-77): deleteRoot/deleteUpdate until the
  * heap is empty or the next deleted batch would not fit in max_keys.  Keys
- * are written in ascending order (HEAP_SORT) to out_dev[0, *n_out).  When
- * n_out is not NULL the call synchronizes the stream to read the count.  A
+ * are written in ascending order (HEAP_SORT) to out_dev[0, *n_out).  No other
+ * operation may use the heap during the call.  When n_out is not NULL the call synchronizes the stream to read the count.  A
  * heap that max_keys holds whole is emptied by one radix sort between its
  * nodes and out_dev (from 4 nodes on; the first bulk operation after
  * gh_heap_restore from 256 on where the batch size has an owner mode) unless an owner depth was

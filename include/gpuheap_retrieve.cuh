@@ -33,7 +33,8 @@
 // block never sees stale L1 lines of a node another block wrote.  Keys are
 // staged in three shared-memory buffers of one batch each; the merges and
 // the sort are the BGPQ heap's (gpuheap_device.cuh: merge path with ties to
-// the first run, bitonic sort), so results equal the reference's.
+// the first run, the sort of an insert batch), so results equal the
+// reference's.
 #pragma once
 #include "gpuheap_device.cuh"
 
