@@ -150,9 +150,8 @@ __device__ __forceinline__ bool wait_for_keys(const H& heap, int* word, const in
 // (a chain) stays with its block, as every hand-over costs a wait.  SSSP,
 // batch 2048 on 24 blocks, exchanging always / with this rule: grid of
 // 2000 x 2000 vertices 1313 / 547 ms (163 / 57 M keys taken), 1000 x 1000
-// 338 / 205; a chain of 20000 158 / 152; R-MAT 18 8.2 / 8.4; 10^5 random
-// vertices of degree 8 (a search of 4 ms) 4.4 / 4.7; four served searches on
-// the 1000 x 1000 grid 188 / 159.
+// 338 / 205; a chain of 20000 158 / 152; R-MAT 18 8.2 / 8.4; four served
+// searches on the 1000 x 1000 grid 188 / 159.
 template <typename H>
 __device__ __forceinline__ bool crowded(const H& heap, int* word, int kept) {
     if (kept <= 8) return false;
