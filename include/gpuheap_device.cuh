@@ -1198,7 +1198,7 @@ struct Heap {
                 const int lim = detail::ld_relaxed(&state->outLimit);
                 c->bc = bc; c->ps = ps; c->dc = dc;
                 const int want = bc > 0 ? batchSize : (PB ? ps : 0);
-                if (want == 0 || (sortOutput && dc + want > lim)) {
+                if (want == 0 || (sortOutput && want > lim - dc)) {  // (dc + want may pass INT_MAX)
                     bulkStop(fair);
                     unlock(0, 0);
                 } else if (bc == 0) {
@@ -1334,7 +1334,7 @@ struct Heap {
                 const int lim = detail::ld_relaxed(&state->outLimit);
                 c->bc = bc; c->ps = ps; c->dc = dc;
                 const int want = bc > 0 ? B : (PB ? ps : 0);
-                if (want == 0 || (sortOutput && dc + want > lim)) {
+                if (want == 0 || (sortOutput && want > lim - dc)) {  // (dc + want may pass INT_MAX)
                     bulkStop(fair);
                     unlock(0, 0);
                 } else if (bc == 0) {
