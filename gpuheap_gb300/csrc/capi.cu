@@ -643,18 +643,19 @@ gh_status gh_heap_sort_host(gh_heap* h, const void* keys_host, long long n, void
     // the copy stream while piece j + 1 is deleted; a heap that one sort
     // empties (k_drain) goes in one piece
     const bool whole = h->d.drain && h->d.ownerDepth < 0 && gh::impl::drains_whole(n, n / B, gh::impl::drain_nodes(h->d));
-    const long long outPiece = whole ? n : piece;
+    const long long outPiece = gh::impl::out_piece(n, piece, B, whole);
     for (long long off = 0; off < n; off += outPiece) {
         const long long len = std::min(outPiece, n - off);
         st = delete_bulk(h, out + off * kb, len, nullptr, nullptr, stream, whole ? n : -1);
         if (st != GH_OK) return st;
-        GH_CUDA(cudaEventRecord(h->sortEv[e], s));
-        GH_CUDA(cudaStreamWaitEvent(c, h->sortEv[e++], 0));
+        cudaEvent_t done = h->sortEv[std::min(e++, 2 * kPieces)];  // a wait keeps the record it met: the last one may serve again
+        GH_CUDA(cudaEventRecord(done, s));
+        GH_CUDA(cudaStreamWaitEvent(c, done, 0));
         GH_CUDA(cudaMemcpyAsync(hout + off * kb, out + off * kb, len * kb, cudaMemcpyDeviceToHost, c));
     }
     // the caller's stream ends after the last copy
-    GH_CUDA(cudaEventRecord(h->sortEv[e], c));
-    GH_CUDA(cudaStreamWaitEvent(s, h->sortEv[e], 0));
+    GH_CUDA(cudaEventRecord(h->sortEv[2 * kPieces + 1], c));
+    GH_CUDA(cudaStreamWaitEvent(s, h->sortEv[2 * kPieces + 1], 0));
     return GH_OK;
 }
 

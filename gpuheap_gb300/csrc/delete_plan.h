@@ -16,5 +16,12 @@ enum class DeletePlan { kAuto, kLoops, kWhole, kPart };
 // pieces, by the loops.  minNodes: drain_nodes().
 inline bool drains_whole(long long keys, long long nodes, int minNodes) { return keys <= INT_MAX && nodes >= minNodes; }
 
+// Keys of each bulk delete that empties a sorted heap of n keys into host
+// memory: all of them, or pieces of whole batches that an int can count.
+inline long long out_piece(long long n, long long piece, int batchSize, bool whole) {
+    const long long most = INT_MAX / batchSize * static_cast<long long>(batchSize);
+    return whole ? n : piece < most ? piece : most;
+}
+
 }  // namespace impl
 }  // namespace gh

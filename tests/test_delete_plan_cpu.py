@@ -17,6 +17,7 @@ int main(int argc, char** argv) {
     long long a[8] = {};
     for (int i = 1; i < argc && i <= 8; ++i) a[i - 1] = std::atoll(argv[i]);
     std::printf("%d\n", drains_whole(a[0], a[1], static_cast<int>(a[2])));
+    if (argc > 4) std::printf("%lld\n", out_piece(a[0], a[3], static_cast<int>(a[4]), false));
 }
 """
 
@@ -40,3 +41,11 @@ def test_one_sort_empties_heaps_of_4_nodes_to_2e31_keys(plan, keys, whole):
     """An output limit is an int: a sort of 2^31 keys and more would not start,
     and gh_heap_sort_host would copy out what its buffer held before."""
     assert plan(keys, keys // 2048, 4) == [whole]
+
+
+@pytest.mark.parametrize("keys,B", [(2**31 - 1, 2048), (2**31, 16), (2**34 + 5, 4096), (2**34 + 2**33, 2048), (2**35, 256)])
+def test_pieces_of_whole_batches_that_an_int_counts(plan, keys, B):
+    piece = -(-(-(-keys // 8)) // B) * B  # an eighth, in whole batches
+    got = plan(keys, keys // B, 4, piece, B)[1]
+    assert got % B == 0 and 0 < got <= 2**31 - 1 and got <= piece
+    assert got == piece or got + B > 2**31 - 1
