@@ -194,7 +194,7 @@ struct ServeDev {
     unsigned long long pad2[15];
     alignas(128) unsigned long long deq;
     unsigned long long pad3[15];
-    alignas(128) unsigned long long admitAt;  // global timer before which no block tries to admit
+    alignas(128) unsigned long long admitAt;  // global timer before which no block tries to admit (raised only; a completion clears it)
     unsigned long long pad4[15];
     // set by the host before the first launch
     alignas(128) ServeReq* ring;  // pinned, ringCap records

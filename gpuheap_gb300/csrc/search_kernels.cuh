@@ -767,13 +767,20 @@ __device__ inline bool try_lock(ServeDev* d) {
     return true;
 }
 
+// Waits for the lock.  Each failed attempt keeps the blocks that look for
+// requests off it for 20 us (the caller lets them on again).  Without that a
+// block that had completed a query met the lock held on every attempt for the
+// whole 2 s, once in some 40000 bursts: an admission every 4.096 us and seven
+// attempts in each, in step.
 __device__ inline bool lock(ServeDev* d) {
     const u64 t0 = gh::detail::globaltimer();
     while (atomicCAS(&d->lock, 0, 1) != 0) {
-        if (gh::detail::globaltimer() - t0 > static_cast<u64>(d->waitNs)) {
+        const u64 now = gh::detail::globaltimer();
+        if (now - t0 > static_cast<u64>(d->waitNs)) {
             fail(d, kServeErrLock);
             return false;
         }
+        atomicMax(&d->admitAt, now + 20000);
         __nanosleep(128);
     }
     __threadfence();
@@ -917,7 +924,7 @@ __device__ inline void admit(ServeDev* d) {
     } else {
         v->idleSince = 0;
     }
-    if (!changed) atomicExch(&d->admitAt, now + 1000);  // nothing new: let the others run for a microsecond
+    if (!changed) atomicMax(&d->admitAt, now + 1000);  // nothing new: let the others run for a microsecond
 }
 
 // Thread 0: the next token for this block, or -1 when the blocks leave.

@@ -44,6 +44,8 @@ modelled here at the level of those atomic steps:
   and search tokens, and the block that retires the last token completes
   the query; requests and completions cross in rings in pinned host memory,
   and the host launches the loop again after an idle exit.
+* the served device loop's lock (`admit`, `complete`): blocks that look for
+  requests stay off it while a completion waits for it.
 * the bulk delete's ticketed turn at node 0 (gpuheap_device.cuh
   `takeTurn`): blocks take node 0 in the order of their tickets.
 * top-down bulk inserts into reserved targets (`insertionReserved`,
@@ -1808,3 +1810,62 @@ def build_model(nodes=6, blocks=2, descending=True):
 
     g0 = BuildState(next=0, lock=(AVAIL,) + (INUSE,) * nodes, heap=(True,) + (False,) * nodes)
     return (g0, (("next", None),) * blocks), [block(i) for i in range(blocks)], final
+
+
+# --------------------------------------------------------------------------
+# the served loop's lock: completions against admissions
+
+ServeLockState = namedtuple("ServeLockState", "lock off waiting admissions")
+
+
+def serve_lock_model(pollers=2, keep_off=True, raise_only=True):
+    """The lock of the served device loop (gpuheap_gb300/csrc/
+    search_kernels.cuh `next_token`, `admit`, `complete`, `lock`).  Idle
+    blocks look for requests under it again and again; a block that has
+    completed a query needs it once.  Timing can let the idle blocks win
+    every race, so the completing block's failed attempts raise `admitAt`,
+    the time before which no idle block tries, and an admission that finds
+    nothing only raises it too; the completion clears it at the end.
+
+    An idle block reads admitAt and then tries the lock, two steps.
+    Invariant: while the completing block waits, each idle block gets the
+    lock at most twice more (it may hold it, and may have read admitAt
+    before it was raised).  Planted: attempts that do not keep the others off
+    (keep_off=False), and admissions that store their own time over the
+    raised one (raise_only=False)."""
+    limit = 2 * pollers
+
+    def completer(g, pc, trace):
+        if pc == "try":
+            if g.lock == 0:
+                return [("takes the lock", _set(g, lock=1, waiting=False), "done")]
+            if g.waiting and (g.off or not keep_off):
+                return []  # another failed attempt changes nothing
+            return [("fails, keeps the others off", _set(g, off=keep_off or g.off, waiting=True), "try")]
+        return [("completes, lets them on, unlocks", _set(g, lock=0, off=False), None)]
+
+    def poller(g, pc, trace):
+        if g.admissions > limit:
+            raise Violation(f"{g.admissions} admissions past a waiting completion", list(trace))
+        if pc == "read":
+            if g.off:
+                return []
+            return [("reads admitAt", g, "cas"), ("no more work", g, None)]
+        if pc == "cas":
+            if g.lock:
+                return [("lock held", g, "read")]
+            return [("takes the lock", _set(g, lock=1, admissions=g.admissions + (1 if g.waiting else 0)), "admit")]
+        return [("finds nothing, unlocks", _set(g, lock=0, off=g.off if raise_only else False), "read")]
+
+    def named(i):
+        def act(g, pc, trace):
+            return poller(g, pc, trace)
+        act.__name__ = f"idle{i}"
+        return act
+
+    def final(g, trace):
+        if g.lock or g.off:
+            raise Violation(f"ended with lock {g.lock}, off {g.off}", trace)
+
+    g0 = ServeLockState(lock=0, off=False, waiting=False, admissions=0)
+    return (g0, ("try",) + ("read",) * pollers), [completer] + [named(i) for i in range(pollers)], final

@@ -1,6 +1,7 @@
 """Protocols of the bulk operations and the searches' exchange, every
 interleaving (oracle/lock_model.py): the last node given back, the end of a
-bulk delete, the locks of the next level, the heap build."""
+bulk delete, the locks of the next level, the heap build; and the served
+loop's lock."""
 import pytest
 
 from oracle import lock_model as lm
@@ -52,3 +53,15 @@ def test_heap_build_finishes(nodes, blocks):
 def test_heap_build_in_ascending_order_deadlocks():
     init, actors, final = lm.build_model(nodes=7, blocks=2, descending=False)
     assert lm.explore(init, actors, final).deadlocks
+
+
+@pytest.mark.parametrize("pollers", [1, 2, 3])
+def test_a_completion_gets_the_served_loops_lock(pollers):
+    finishes(lm.serve_lock_model(pollers=pollers))
+
+
+@pytest.mark.parametrize("mistake", [dict(keep_off=False), dict(raise_only=False)])
+def test_admissions_that_pass_a_waiting_completion_are_caught(mistake):
+    init, actors, final = lm.serve_lock_model(**mistake)
+    with pytest.raises(lm.Violation, match="past a waiting completion"):
+        lm.explore(init, actors, final)
